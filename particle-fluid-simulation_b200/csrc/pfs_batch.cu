@@ -37,15 +37,24 @@ struct Scene {
     uint32_t off, n;
     pfs_params params;
     DevParams dp;
+    double fluid;  // volume its particles fill (fluid_volume)
 };
 
-// Spatial-order buckets a batch reserves per particle and per scene: the
-// cap a world uses (derive_params: max(4 n, 4096) blocks), so a scene's
-// grid search reads the same blocks (single cells where they fit) as the
-// scene's own world.  Coarser blocks made the gather test up to several
-// times as many candidates.
-constexpr uint32_t kBlocksPerParticle = 4;
+// Spatial-order buckets a batch reserves per particle and per scene: about the
+// cap a world uses (derive_params), so a scene's grid search reads single cells
+// where its own world does.  Coarser buckets send the scene to the
+// one-warp-per-particle pass.
+constexpr uint32_t kBlocksPerParticle = 16;
 constexpr uint32_t kBlocksPerScene = 4096;
+// Scenes' buckets start at multiples of this (k_bucket_alloc's thread block).
+constexpr uint32_t kBlockAlign = 256;
+// Particles per block of a batch's scenes: there are scenes enough to fill the
+// device with full blocks.
+constexpr uint32_t kBlockMembers = 104;
+
+uint32_t batch_blocks(uint32_t max_particles, uint32_t max_scenes) {
+    return kBlocksPerParticle * max_particles + (kBlocksPerScene + kBlockAlign) * max_scenes;
+}
 
 __global__ void k_fill_sid(uint32_t n, const uint32_t* __restrict__ offs, uint32_t scenes,
                            uint32_t* __restrict__ sid) {
@@ -108,6 +117,7 @@ size_t batch_arena_bytes(uint32_t cap_n, uint32_t cap_s, int precision, uint32_t
     size_t b = world_arena_bytes(cap_n, 0, precision, blocks_cap, NLIST_CAP_MAX, 0);
     b += (size_t)cap_s * sizeof(DevParams) + (size_t)cap_n * 4 /*sid*/ + ((size_t)cap_s + 1) * 4;
     b += 2 * (size_t)cap_n * 16; /* x0 v0 */
+    b += ((size_t)blocks_cap / 256 + 1) * 4; /* cvshift */
     return b + 8 * 256;
 }
 
@@ -125,7 +135,8 @@ DevParams global_params(uint32_t n, uint32_t blocks) {
 // them, refill the per-slot scene ids and recompute all keys.
 int repack_tables(pfs_batch* B) {
     uint32_t block_base = 0;
-    uint32_t geo_any = 0;
+    uint32_t geo_any = 0, all_geo = 1, entries = 0;
+    std::vector<uint32_t> vshift;
     std::vector<DevParams> dps(B->scenes.size());
     std::vector<uint32_t> offs(B->scenes.size() + 1);
     for (size_t k = 0; k < B->scenes.size(); k++) {
@@ -135,8 +146,12 @@ int repack_tables(pfs_batch* B) {
         d.key_base = s.off;
         d.block_base = block_base;
         d.list_cap = NLIST_CAP_MAX;
-        block_base += spatial_blocks(d);
+        block_base += (spatial_blocks(d) + kBlockAlign - 1) / kBlockAlign * kBlockAlign;
         geo_any |= d.geo;
+        all_geo &= d.geo;
+        if (d.geo)
+            entries = std::max(entries, cells_entries(&d, cell_density(d, s.params, s.n, s.fluid)));
+        vshift.resize(block_base / kBlockAlign, d.geo ? (uint32_t)(d.bsx + d.bsy + d.bsz) : 32u);
         dps[k] = d;
         offs[k] = s.off;
     }
@@ -144,8 +159,12 @@ int repack_tables(pfs_batch* B) {
     if (block_base > B->blocks_cap) return PFS_ERANGE;  // cannot happen: blocks are capped per scene
     B->b.nblocks = block_base;
     B->b.geo_any = geo_any;
+    B->b.all_geo = all_geo;
+    B->b.cells_entries = entries;
     cudaError_t e = cudaSuccess;
-    if (!dps.empty())
+    if (!vshift.empty())
+        e = cudaMemcpyAsync(B->b.cvshift, vshift.data(), vshift.size() * 4, cudaMemcpyHostToDevice, B->stream);
+    if (e == cudaSuccess && !dps.empty())
         e = cudaMemcpyAsync(B->d_scenes, dps.data(), dps.size() * sizeof(DevParams),
                             cudaMemcpyHostToDevice, B->stream);
     if (e == cudaSuccess && B->n_total) {
@@ -210,7 +229,7 @@ Scene* find_scene(pfs_batch* B, int32_t id, size_t* index = nullptr) {
 extern "C" {
 
 uint64_t pfs_batch_bytes(uint32_t max_particles, uint32_t max_scenes, int32_t precision) {
-    const uint32_t blocks = kBlocksPerParticle * max_particles + kBlocksPerScene * max_scenes;
+    const uint32_t blocks = batch_blocks(max_particles, max_scenes);
     return batch_arena_bytes(max_particles, max_scenes, precision, blocks);
 }
 
@@ -231,7 +250,7 @@ int pfs_batch_create(uint32_t max_particles, uint32_t max_scenes, int32_t precis
     B->cap_s = max_scenes;
     B->precision = precision;
     B->substeps = substeps;
-    B->blocks_cap = kBlocksPerParticle * max_particles + kBlocksPerScene * max_scenes;
+    B->blocks_cap = batch_blocks(max_particles, max_scenes);
     cudaError_t e = cudaStreamCreateWithFlags(&B->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess)
         e = B->arena.reserve(batch_arena_bytes(max_particles, max_scenes, precision, B->blocks_cap));
@@ -267,6 +286,8 @@ int pfs_batch_create(uint32_t max_particles, uint32_t max_scenes, int32_t precis
     b.ncount = (int32_t*)a.take(u);
     b.scanq = (uint32_t*)a.take(u);
     b.scanq_n = (uint32_t*)a.take(256);
+    b.clist = (uint32_t*)a.take(u);
+    b.cvshift = (uint32_t*)a.take(((size_t)B->blocks_cap / 256 + 1) * 4);
     B->d_scenes = (DevParams*)a.take((size_t)max_scenes * sizeof(DevParams));
     B->d_sid = (uint32_t*)a.take(u);
     B->d_offs = (uint32_t*)a.take(((size_t)max_scenes + 1) * 4);
@@ -278,7 +299,7 @@ int pfs_batch_create(uint32_t max_particles, uint32_t max_scenes, int32_t precis
     bool ok = b.x && b.v && b.xs && b.vs && b.xp && b.vp && b.rr && b.keys && b.skeys && b.perm &&
               b.keys_tmp && b.vals_tmp && b.sort_scratch && b.table && b.err && b.order &&
               b.bucket && b.brank && b.bcount && b.boffset && b.bcounter && b.nlist && b.ncount &&
-              b.scanq && b.scanq_n && B->d_scenes && B->d_sid && B->d_offs && B->x0 && B->v0;
+              b.scanq && b.scanq_n && b.clist && b.cvshift && B->d_scenes && B->d_sid && B->d_offs && B->x0 && B->v0;
     if (ok && precision == PFS_FP16_CELL) ok = fp16_carve(a, max_particles, &B->h16);
     if (!ok) {
         pfs_batch_destroy(B);
@@ -309,7 +330,8 @@ int pfs_batch_add_scene(pfs_batch* B, const pfs_params* p, uint32_t n, const flo
     s.off = B->n_total;
     s.n = n;
     s.params = *p;
-    derive_params(*p, n, &s.dp);
+    s.fluid = fluid_volume(*p, n, pos4);
+    derive_params(*p, n, &s.dp, -1, s.fluid, kBlockMembers);
     fit_spatial_blocks(&s.dp, std::max(kBlocksPerParticle * n, kBlocksPerScene));
     const size_t f4 = (size_t)n * 16;
     cudaError_t e = cudaMemcpyAsync(B->b.x + s.off, pos4, f4, cudaMemcpyDefault, B->stream);
@@ -486,7 +508,7 @@ static int batch_apply_shape(pfs_batch* B, int32_t shape, int32_t search) {
     if (shape < NBR_SIMPLE || shape > NBR_FLAT || search < -1 || search > 1) return PFS_EINVAL;
     B->b.variant = shape;
     for (Scene& s : B->scenes) {
-        derive_params(s.params, s.n, &s.dp, search);
+        derive_params(s.params, s.n, &s.dp, search, s.fluid, kBlockMembers);
         fit_spatial_blocks(&s.dp, std::max(kBlocksPerParticle * s.n, kBlocksPerScene));
     }
     B->layout_dirty = true;

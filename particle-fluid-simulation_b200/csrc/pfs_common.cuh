@@ -38,11 +38,18 @@ struct DevParams {
     uint32_t n;
     int32_t flags;
     // spatial processing order of the neighbour passes: x* cells clamped to
-    // [0, ng?-1] are grouped into blocks of 2^bshift cells per axis, nb? blocks
-    // per axis (row-major block id)
+    // [0, ng?-1] fall into buckets of 2^cshift cells per axis; buckets are
+    // grouped into blocks of 2^bsx x 2^bsy x 2^bsz, nb? blocks per axis, and
+    // numbered block by block (blocks row-major), so a block's buckets are
+    // consecutive
     uint32_t ngx, ngy, ngz;
     uint32_t nbx, nby, nbz;
-    int32_t bshift;
+    int32_t cshift, bsx, bsy, bsz;
+    // cell-grouped density pass (pfs_cells.cuh): neighbourhood layers staged at a
+    // time, and the distance from a cell face, in cells, within which rounding
+    // could hide a neighbour two cells away
+    int32_t blayers;
+    float edge;
     // batched scenes: the scene's slice of the shared key space (table slots
     // key_base .. key_base + mask) and of the spatial-order blocks; 0 for a
     // world.  n is the particle count of the whole table either way.
@@ -84,7 +91,15 @@ __device__ __forceinline__ DevParams params_of(const DevParams& P0, const SceneR
     }
 }
 
-// Block (bucket) of a predicted position for the spatial processing order.
+// Spatial-order bucket of bucket coordinates (cells >> cshift).
+__device__ __forceinline__ uint32_t spatial_id(const DevParams& P, uint32_t x, uint32_t y, uint32_t z) {
+    const uint32_t blk = (x >> P.bsx) + P.nbx * ((y >> P.bsy) + P.nby * (z >> P.bsz));
+    const uint32_t in = (x & ((1u << P.bsx) - 1u)) |
+                        ((y & ((1u << P.bsy) - 1u)) | (z & ((1u << P.bsz) - 1u)) << P.bsy) << P.bsx;
+    return P.block_base + ((blk << (P.bsx + P.bsy + P.bsz)) | in);
+}
+
+// Bucket of a predicted position for the spatial processing order.
 __device__ __forceinline__ uint32_t spatial_block(const DevParams& P, float x, float y, float z) {
     int32_t cx = __float2int_rz(floorf(__fdiv_rn(__fsub_rn(x, P.minx), P.h)));
     int32_t cy = __float2int_rz(floorf(__fdiv_rn(__fsub_rn(y, P.miny), P.h)));
@@ -92,9 +107,7 @@ __device__ __forceinline__ uint32_t spatial_block(const DevParams& P, float x, f
     cx = min(max(cx, 0), (int32_t)P.ngx - 1);
     cy = min(max(cy, 0), (int32_t)P.ngy - 1);
     cz = min(max(cz, 0), (int32_t)P.ngz - 1);
-    const uint32_t bx = (uint32_t)cx >> P.bshift, by = (uint32_t)cy >> P.bshift,
-                   bz = (uint32_t)cz >> P.bshift;
-    return P.block_base + bx + P.nbx * (by + P.nby * bz);
+    return spatial_id(P, (uint32_t)cx >> P.cshift, (uint32_t)cy >> P.cshift, (uint32_t)cz >> P.cshift);
 }
 
 // Bucket of the spatial processing order: the block of x* (spatial_block),
@@ -114,6 +127,11 @@ __device__ __forceinline__ uint32_t spatial_bucket(const DevParams& P, float x, 
     const uint32_t blk = bx + P.nsx * (by + P.nsy * bz);
     return (blk << (P.sbx + P.sby + P.sbz)) | lx | (ly << P.sbx) | (lz << (P.sbx + P.sby));
 }
+
+// Entries the cell-grouped density pass stages at a time: 17 KB, so that several
+// thread blocks share an SM; more only where one layer of one cell needs it.
+constexpr uint32_t CELLS_STAGE = 1088;
+constexpr uint32_t CELLS_STAGE_MAX = 2048;
 
 #define PFS_ADD(a, b) __fadd_rn((a), (b))
 #define PFS_SUB(a, b) __fsub_rn((a), (b))
@@ -220,13 +238,24 @@ __device__ __forceinline__ float4 speed_color(float3 v) {
 // Host: derive DevParams from pfs_params (same arithmetic as the oracle's
 // pfso_derive, which the GPU parity tests rely on).
 // search: -1 automatic (or PFS_NEIGHBOR_SEARCH), 0 table scan, 1 grid search
-// (where the grid bound allows it).
-void derive_params(const pfs_params& p, uint32_t n, DevParams* out, int search = -1);
+// (where the grid bound allows it).  fluid: volume the particles fill (0:
+// unknown), from which the blocks of the grid search are sized; members:
+// particles per block to aim for (0: by n).
+void derive_params(const pfs_params& p, uint32_t n, DevParams* out, int search = -1, double fluid = 0.0,
+                   uint32_t members = 0);
+// Volume of the bounding box of a sample of an initial state's particles inside
+// the world box (0 for device memory).
+double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4);
+// Particles per cell where the fluid is.
+double cell_density(const DevParams& P, const pfs_params& p, uint32_t n, double fluid);
+// Entries the cell-grouped density pass stages at a time for P's blocks at this
+// many particles per cell; sets P->blayers.
+uint32_t cells_entries(DevParams* P, double per_cell);
 // The grid search is possible for this table and box.
 bool grid_search_allowed(const pfs_params& p, uint32_t n);
 // Buckets of the spatial processing order.
 uint32_t spatial_blocks(const DevParams& P);
-// Coarsen the spatial-order blocks until at most `cap` remain.
+// Coarsen the spatial order until at most `cap` buckets remain.
 void fit_spatial_blocks(DevParams* P, uint32_t cap);
 
 }  // namespace pfs

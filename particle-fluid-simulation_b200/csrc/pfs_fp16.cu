@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include "pfs_common.cuh"
+#include "pfs_cells.cuh"
 #include "pfs_flat.cuh"
 #include "pfs_fp16.cuh"
 #include "pfs_geo.cuh"
@@ -63,6 +64,13 @@ __device__ __forceinline__ void dens16_terms(float q2, float& a2, float& a3) {
     const float a = 1.0f - q;
     a2 = a * a;
     a3 = a2 * a;
+}
+
+__device__ __forceinline__ float2 density16_finish(const DevParams& P, float s2, float s3) {
+    const float h = P.h, h2 = h * h;
+    const float d = (P.m * (s2 * h2)) / P.volume;
+    const float nd = (P.m * (s3 * h2 * h)) * P.near_inv;
+    return make_float2((0.01f < d) ? d : 0.01f, (0.01f < nd) ? nd : 0.01f);
 }
 
 // ---- flat shape of the FP16-cell density pass -------------------------------
@@ -183,14 +191,49 @@ k_density16_flat(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const
     const bool scan = live && (over || !((meta & FLAT_LIST_OK) != 0 && cnt <= (int32_t)P.list_cap));
     if (live) {
         if (over) density16_scan_one(P, xp[i], me, rec, table, n, err, s2, c2, s3, c3);
-        const float h = P.h, h2 = h * h;
-        const float d = (P.m * (s2 * h2)) / P.volume;
-        const float nd = (P.m * (s3 * h2 * h)) * P.near_inv;
-        rr[i] = make_float2((0.01f < d) ? d : 0.01f, (0.01f < nd) ? nd : 0.01f);
+        rr[i] = density16_finish(P, s2, s3);
         ncount[t] = scan ? -1 : cnt;
     }
     flat_enqueue(scan, t, scanq, scanq_n);
 }
+
+// ---- grid search: the cell-grouped pass (pfs_cells.cuh) over the records ------
+
+struct Dens16 {
+    const uint4* __restrict__ rec;
+    __device__ __forceinline__ float3 self(const float4* __restrict__, uint32_t i) const {
+        const Unpacked u = rec_unpack(rec[i]);
+        return make_float3(u.px, u.py, u.pz);
+    }
+    __device__ __forceinline__ float4 stage(uint32_t j) const {
+        const Unpacked u = rec_unpack(__ldg(rec + j));
+        return make_float4(u.px, u.py, u.pz, __uint_as_float(j));
+    }
+    // of a candidate and a particle given by its negated position, in units of h
+    __device__ __forceinline__ float dist2(const float4 c, float nx, float ny, float nz) const {
+        const float ex = c.x + nx, ey = c.y + ny, ez = c.z + nz;
+        return fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+    }
+    __device__ __forceinline__ void dist2_pair(f32x2 x, f32x2 y, f32x2 z, f32x2 nx, f32x2 ny, f32x2 nz, float& a,
+                                               float& b) const {
+        const f32x2 ex = add2(x, nx), ey = add2(y, ny), ez = add2(z, nz);
+        unpack2(fma2(ex, ex, fma2(ey, ey, mul2(ez, ez))), a, b);
+    }
+    __device__ __forceinline__ bool in_reach(float q2, float) const { return q2 < 1.0f; }
+    __device__ __forceinline__ void terms(const DevParams&, float q2, float& a2, float& a3) const {
+        dens16_terms(q2, a2, a3);
+    }
+    struct Sum {
+        float s2 = 0.0f, c2 = 0.0f, s3 = 0.0f, c3 = 0.0f;
+        __device__ __forceinline__ void add(bool take, float a2, float a3) {
+            if (take) {
+                kahan(s2, c2, a2);
+                kahan(s3, c3, a3);
+            }
+        }
+        __device__ __forceinline__ float2 finish(const DevParams& P) const { return density16_finish(P, s2, s3); }
+    };
+};
 
 // Particle-side constants of the force terms in the units of the records.
 struct Self16 {
@@ -378,20 +421,15 @@ k_force16(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const float4
 constexpr int GEO16_DCAP = 512;
 constexpr int GEO16_FCAP = 256;
 
-__device__ __forceinline__ bool geo16_skip(const DevParams& P0, SceneRef sr, uint32_t i, bool batch) {
-    return batch ? !__ldg(&sr.scenes[__ldg(sr.sid + i)].geo) : !P0.geo;
-}
-
-// Density pass of the grid-search particles, as k_density16_flat (same sums in
-// the same order, same list and queue decisions).  Nine blocks per SM, as
-// k_density_geo.
+// Density pass of the grid-search particles the cell-grouped pass leaves
+// (slowq): same sums in the same order, same list and queue decisions.  Nine
+// blocks per SM, as k_density_geo.
 template <bool BATCH>
 __global__ void __launch_bounds__(GEO_WARPS * 32, 9)
 k_density16_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const uint4* __restrict__ rec,
                 const int2* __restrict__ table, const uint32_t* __restrict__ order,
-                const uint32_t* __restrict__ bucket, const uint32_t* __restrict__ brank,
                 const uint32_t* __restrict__ bcount, const uint32_t* __restrict__ boffset,
-                uint32_t nblocks, float2* __restrict__ rr, int32_t* __restrict__ nlist,
+                const uint32_t* __restrict__ slowq, float2* __restrict__ rr, int32_t* __restrict__ nlist,
                 int32_t* __restrict__ ncount, uint32_t* __restrict__ scanq,
                 uint32_t* __restrict__ scanq_n, uint32_t* __restrict__ err) {
     __shared__ int32_t s_j[GEO_WARPS][GEO16_DCAP];
@@ -403,8 +441,14 @@ k_density16_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const 
     float* sa = s_a[w];
     float* sb = s_b[w];
     const uint32_t n = P0.n;
-    for (uint32_t i = blockIdx.x * GEO_WARPS + w; i < n; i += gridDim.x * GEO_WARPS) {
-        if (geo16_skip(P0, sr, i, BATCH)) continue;
+    const uint32_t total_q = min(scanq_n[CTR_SLOW], n);
+    for (uint32_t q = blockIdx.x * GEO_WARPS + w; q < total_q; q += gridDim.x * GEO_WARPS) {
+        const uint32_t t = slowq[q];
+        const uint32_t i = t < n ? order[t] : n;
+        if (i >= n) {
+            if (lane == 0) atomicOr(err, ERR_PERM_RANGE);
+            continue;
+        }
         const DevParams P = params_of<BATCH>(P0, sr, i);
         const float4 sp = xp[i];
         const Unpacked me = rec_unpack(rec[i]);
@@ -454,7 +498,6 @@ k_density16_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const 
                                   });
         float s2 = 0.0f, c2 = 0.0f, s3 = 0.0f, c3 = 0.0f;  // lane 0: s2 c2, lane 1: s3 c3
         int32_t cnt = 0;
-        const uint32_t t = order_position(i, n, nblocks, bucket, brank, boffset);
         if (m <= GEO16_DCAP) {
             warp_sort(sj, m);
             for (int k = lane; k < m; k += 32) {
@@ -506,7 +549,7 @@ k_density16_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const 
                         const bool e = j != (int32_t)i;
                         const uint32_t mk = __ballot_sync(full, e);
                         const int32_t pos = cnt + __popc(mk & lt);
-                        if (e && pos < (int32_t)P.list_cap && t < n) nlist[(size_t)pos * n + t] = j;
+                        if (e && pos < (int32_t)P.list_cap) nlist[(size_t)pos * n + t] = j;
                         cnt += __popc(mk);
                     }
                 }
@@ -551,19 +594,12 @@ k_density16_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const 
         s2 = __shfl_sync(full, s2, 0);
         s3 = __shfl_sync(full, s3, 1);
         if (lane == 0) {
-            const float h2 = h * h;
-            const float dn = (P.m * (s2 * h2)) / P.volume;
-            const float nd = (P.m * (s3 * h2 * h)) * P.near_inv;
-            rr[i] = make_float2((0.01f < dn) ? dn : 0.01f, (0.01f < nd) ? nd : 0.01f);
-            if (t < n) {
-                const bool scan = !(list_ok && cnt <= (int32_t)P.list_cap);
-                ncount[t] = scan ? -1 : cnt;
-                if (scan) {
-                    const uint32_t q = atomicAdd(scanq_n + 1, 1u);
-                    if (q < n) *geo_queue_entry(scanq, n, q) = i;
-                }
-            } else {
-                atomicOr(err, ERR_PERM_RANGE);
+            rr[i] = density16_finish(P, s2, s3);
+            const bool scan = !(list_ok && cnt <= (int32_t)P.list_cap);
+            ncount[t] = scan ? -1 : cnt;
+            if (scan) {
+                const uint32_t k = atomicAdd(scanq_n + CTR_GEOQ, 1u);
+                if (k < n) *geo_queue_entry(scanq, n, k) = i;
             }
         }
         __syncwarp();
@@ -725,21 +761,18 @@ cudaError_t launch_density_fp16(const DevParams& P, const StepBuffers& b, const 
                                 cudaStream_t s) {
     if (P.n == 0) return cudaSuccess;
     const unsigned g = grid_for(P.n, NBR_THREADS);
-    if (b.sr.scenes)
-        k_density16_flat<true><<<g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, f.rec, b.table, b.order, b.rr,
-                                                          b.nlist, b.ncount, b.scanq, b.scanq_n, b.err);
-    else
-        k_density16_flat<false><<<g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, f.rec, b.table, b.order, b.rr,
-                                                           b.nlist, b.ncount, b.scanq, b.scanq_n, b.err);
+    if (!b.all_geo) {
+        auto k = b.sr.scenes ? k_density16_flat<true> : k_density16_flat<false>;
+        k<<<g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, f.rec, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
+                                    b.scanq_n, b.err);
+    }
     if (b.geo_any) {
-                if (b.sr.scenes)
-            k_density16_geo<true><<<geo16_grid(k_density16_geo<true>, P.n), GEO_WARPS * 32, 0, s>>>(
-                P, b.sr, b.xp, f.rec, b.table, b.order, b.bucket, b.brank, b.bcount, b.boffset,
-                b.nblocks, b.rr, b.nlist, b.ncount, b.scanq, b.scanq_n, b.err);
-        else
-            k_density16_geo<false><<<geo16_grid(k_density16_geo<false>, P.n), GEO_WARPS * 32, 0, s>>>(
-                P, b.sr, b.xp, f.rec, b.table, b.order, b.bucket, b.brank, b.bcount, b.boffset,
-                b.nblocks, b.rr, b.nlist, b.ncount, b.scanq, b.scanq_n, b.err);
+        const cudaError_t e = launch_cells(P, b, Dens16{f.rec}, s);
+        if (e != cudaSuccess) return e;
+        auto k = b.sr.scenes ? k_density16_geo<true> : k_density16_geo<false>;
+        k<<<geo16_grid(k, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, f.rec, b.table, b.order, b.bcount, b.boffset,
+                                                        b.keys_tmp, b.rr, b.nlist, b.ncount, b.scanq, b.scanq_n,
+                                                        b.err);
     }
     return cudaGetLastError();
 }

@@ -9,7 +9,8 @@
 //
 // The grid search finds the same in-range candidates through the spatial
 // grid of x* the reorder already builds (order / bcount / boffset: slots
-// bucketed by block of 2^bshift cells of x*), sorts them by slot, and then
+// bucketed by cell of x*, coarser where the buffers do not hold single cells),
+// sorts them by slot, and then
 // walks the 27 table ranges exactly as the scan does, taking from each range
 // [start, end) only its in-range members, in slot order.  The lanes of a warp
 // gather, sort and evaluate the terms in parallel; the per-particle sums are
@@ -64,7 +65,7 @@ __device__ __forceinline__ int warp_gather(const DevParams& P, float x, float y,
                                            int cap, uint32_t* __restrict__ err, Test&& test) {
     const int lane = threadIdx.x & 31;
     const uint32_t n = P.n;
-    const uint32_t sh = (uint32_t)P.bshift;
+    const uint32_t sh = (uint32_t)P.cshift;
     uint32_t x0, x1, y0, y1, z0, z1;
     geo_axis(x, P.minx, P.h, P.ngx, sh, x0, x1);
     geo_axis(y, P.miny, P.h, P.ngy, sh, y0, y1);
@@ -78,7 +79,7 @@ __device__ __forceinline__ int warp_gather(const DevParams& P, float x, float y,
         uint32_t c = 0, o = 0;
         if (b < nb) {
             const uint32_t bx = x0 + b % wx, by = y0 + (b / wx) % wy, bz = z0 + b / (wx * wy);
-            const uint32_t blk = P.block_base + bx + P.nbx * (by + P.nby * bz);
+            const uint32_t blk = spatial_id(P, bx, by, bz);
             c = __ldg(bcount + blk);
             if (c) {
                 o = __ldg(boffset + blk);
@@ -159,8 +160,11 @@ __device__ __forceinline__ void warp_sort(int32_t* s_j, int m) {
 // GEO_CHUNK items from a counter the reorder zeroes each substep (lane 0
 // adds, the warp shares the result).  Particles of dense scenes cost many
 // times those of sparse ones, so the warps of a batch take work as they free
-// up instead of a fixed stride of it.  Called by all 32 lanes.
-constexpr uint32_t GEO_CHUNK = 4;
+// up instead of a fixed stride of it.  One at a time: the queues are short (a
+// few of each thousand particles), and one warp taking four of them in turn was
+// most of the pass (300,000 particles, 85 queued: 0.58 ms).  Called by all 32
+// lanes.
+constexpr uint32_t GEO_CHUNK = 1;
 __device__ __forceinline__ uint32_t warp_take(uint32_t* ctr) {
     uint32_t base = 0;
     if ((threadIdx.x & 31) == 0) base = atomicAdd(ctr, GEO_CHUNK);
@@ -178,17 +182,6 @@ __device__ __forceinline__ int geo_lower(const int32_t* a, int m, int32_t key) {
             hi = mid;
     }
     return lo;
-}
-
-// Position of slot i in the processing order (n when its block is invalid).
-__device__ __forceinline__ uint32_t order_position(uint32_t i, uint32_t n, uint32_t nblocks,
-                                                   const uint32_t* __restrict__ bucket,
-                                                   const uint32_t* __restrict__ brank,
-                                                   const uint32_t* __restrict__ boffset) {
-    const uint32_t blk = __ldg(bucket + i);
-    if (blk >= nblocks) return n;
-    const uint32_t t = __ldg(boffset + blk) + __ldg(brank + i);
-    return t < n ? t : n;
 }
 
 // Queue of grid-search particles whose force pass must evaluate in full: it

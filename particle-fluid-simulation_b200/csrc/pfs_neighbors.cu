@@ -40,6 +40,7 @@
 #include <cuda_runtime.h>
 
 #include "pfs_common.cuh"
+#include "pfs_cells.cuh"
 #include "pfs_flat.cuh"
 #include "pfs_geo.cuh"
 #include "pfs_nbr.cuh"
@@ -500,6 +501,56 @@ k_density_flat(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const i
     flat_enqueue(scan, t, scanq, scanq_n);
 }
 
+// ---- grid search: the cell-grouped pass (pfs_cells.cuh) ----------------------
+
+struct Dens32 {
+    const float4* __restrict__ xp;
+    __device__ __forceinline__ float3 self(const float4* __restrict__ x, uint32_t i) const {
+        const float4 p = x[i];
+        return make_float3(p.x, p.y, p.z);
+    }
+    __device__ __forceinline__ float4 stage(uint32_t j) const {
+        const float4 p = __ldg(xp + j);
+        return make_float4(p.x, p.y, p.z, __uint_as_float(j));
+    }
+    // of a candidate and a particle given by its negated position
+    __device__ __forceinline__ float dist2(const float4 c, float nx, float ny, float nz) const {
+        const float d0 = PFS_ADD(c.x, nx), d1 = PFS_ADD(c.y, ny), d2 = PFS_ADD(c.z, nz);
+        return PFS_ADD(PFS_ADD(PFS_MUL(d0, d0), PFS_MUL(d1, d1)), PFS_MUL(d2, d2));
+    }
+    // of two candidates at once.  The sums are not packed: ptxas contracts a packed
+    // multiply and a packed add into a fused one, whatever rounding they ask for.
+    __device__ __forceinline__ void dist2_pair(f32x2 x, f32x2 y, f32x2 z, f32x2 nx, f32x2 ny, f32x2 nz, float& a,
+                                               float& b) const {
+        const f32x2 d0 = add2(x, nx), d1 = add2(y, ny), d2 = add2(z, nz);
+        float ax, ay, az, bx, by, bz;
+        unpack2(mul2(d0, d0), ax, bx);
+        unpack2(mul2(d1, d1), ay, by);
+        unpack2(mul2(d2, d2), az, bz);
+        a = PFS_ADD(PFS_ADD(ax, ay), az);
+        b = PFS_ADD(PFS_ADD(bx, by), bz);
+    }
+    __device__ __forceinline__ bool in_reach(float dd, float skip) const { return dd < skip; }
+    // density_term's increments; adding them in order gives its sums
+    __device__ __forceinline__ void terms(const DevParams& P, float dd, float& t, float& tn) const {
+        const float a = PFS_SUB(P.h, PFS_SQRT(dd));
+        const float a2 = PFS_MUL(a, a);
+        t = PFS_MUL(P.m, a2);
+        tn = PFS_MUL(P.m, PFS_MUL(a2, a));
+    }
+    struct Sum {
+        float total = 0.0f, total_near = 0.0f;
+        // (adding +0 changes neither sum: they start at +0)
+        __device__ __forceinline__ void add(bool take, float t, float tn) {
+            total = PFS_ADD(total, take ? t : 0.0f);
+            total_near = PFS_ADD(total_near, take ? tn : 0.0f);
+        }
+        __device__ __forceinline__ float2 finish(const DevParams& P) const {
+            return density_finish(P, total, total_near);
+        }
+    };
+};
+
 // ---- grid search (pfs_geo.cuh): one warp per particle ------------------------
 
 // In-range candidates a warp holds per particle (beyond them it walks the
@@ -555,23 +606,17 @@ __device__ __forceinline__ float force_chain_add(float acc, int lane, const floa
     return PFS_ADD(acc, inc[lane][k]);
 }
 
-__device__ __forceinline__ bool geo_skip(const DevParams& P0, SceneRef sr, uint32_t i, bool batch) {
-    return batch ? !__ldg(&sr.scenes[__ldg(sr.sid + i)].geo) : !P0.geo;
-}
-
-// Density pass of the grid-search particles: warp w walks slots w, w + W, ...
-// and handles those whose scene uses the grid search.  Same sums, list and
-// queue decisions as k_density_list; particles it cannot list go to the
-// grid-search queue.  Nine blocks of 24 KB fill an SM's shared memory; the
+// Density pass of the grid-search particles the cell-grouped pass leaves (slowq,
+// positions in the processing order).  Same sums, list and queue decisions as
+// k_density_list; particles it cannot list go to the grid-search queue.  Nine blocks of 24 KB fill an SM's shared memory; the
 // register cap of 56 per thread lets the batch form (per-scene parameters)
 // keep all nine resident as well.
 template <bool BATCH>
 __global__ void __launch_bounds__(GEO_WARPS * 32, 9)
 k_density_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const int2* __restrict__ table,
-              const uint32_t* __restrict__ order, const uint32_t* __restrict__ bucket,
-              const uint32_t* __restrict__ brank, const uint32_t* __restrict__ bcount,
-              const uint32_t* __restrict__ boffset, uint32_t nblocks, float2* __restrict__ rr,
-              int32_t* __restrict__ nlist, int32_t* __restrict__ ncount, uint32_t* __restrict__ scanq,
+              const uint32_t* __restrict__ order, const uint32_t* __restrict__ bcount,
+              const uint32_t* __restrict__ boffset, const uint32_t* __restrict__ slowq,
+              float2* __restrict__ rr, int32_t* __restrict__ nlist, int32_t* __restrict__ ncount, uint32_t* __restrict__ scanq,
               uint32_t* __restrict__ scanq_n, uint32_t* __restrict__ err) {
     __shared__ int32_t s_j[GEO_WARPS][GEO_DCAP];
     __shared__ float s_a[GEO_WARPS][GEO_DCAP];
@@ -582,9 +627,15 @@ k_density_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const in
     float* sa = s_a[w];
     float* sb = s_b[w];
     const uint32_t n = P0.n;
-    for (uint32_t base = warp_take(scanq_n + 2); base < n; base = warp_take(scanq_n + 2))
-    for (uint32_t i = base; i < min(base + GEO_CHUNK, n); i++) {
-        if (geo_skip(P0, sr, i, BATCH)) continue;
+    const uint32_t total_q = min(scanq_n[CTR_SLOW], n);
+    for (uint32_t base = warp_take(scanq_n + CTR_SLOWWORK); base < total_q; base = warp_take(scanq_n + CTR_SLOWWORK))
+    for (uint32_t q = base; q < min(base + GEO_CHUNK, total_q); q++) {
+        const uint32_t t = slowq[q];
+        const uint32_t i = t < n ? order[t] : n;
+        if (i >= n) {
+            if (lane == 0) atomicOr(err, ERR_PERM_RANGE);
+            continue;
+        }
         const DevParams P = params_of<BATCH>(P0, sr, i);
         const float4 sp = xp[i];
         const float h = P.h, skip = P.skip_d2;
@@ -634,7 +685,6 @@ k_density_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const in
                                   });
         float total = 0.0f, total_near = 0.0f;
         int32_t cnt = 0;
-        const uint32_t t = order_position(i, n, nblocks, bucket, brank, boffset);
         if (m <= GEO_DCAP) {
             warp_sort(sj, m);
             for (int k = lane; k < m; k += 32) {
@@ -686,7 +736,7 @@ k_density_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const in
                         const bool e = j != (int32_t)i;
                         const uint32_t mk = __ballot_sync(full, e);
                         const int32_t pos = cnt + __popc(mk & lt);
-                        if (e && pos < (int32_t)P.list_cap && t < n) __stcs(nlist + (size_t)pos * n + t, j);
+                        if (e && pos < (int32_t)P.list_cap) __stcs(nlist + (size_t)pos * n + t, j);
                         cnt += __popc(mk);
                     }
                 }
@@ -735,15 +785,11 @@ k_density_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const in
         total_near = __shfl_sync(full, total_near, 1);
         if (lane == 0) {
             rr[i] = density_finish(P, total, total_near);
-            if (t < n) {
-                const bool scan = !(list_ok && cnt <= (int32_t)P.list_cap);
-                ncount[t] = scan ? -1 : cnt;
-                if (scan) {
-                    const uint32_t q = atomicAdd(scanq_n + 1, 1u);
-                    if (q < n) *geo_queue_entry(scanq, n, q) = i;
-                }
-            } else {
-                atomicOr(err, ERR_PERM_RANGE);
+            const bool scan = !(list_ok && cnt <= (int32_t)P.list_cap);
+            ncount[t] = scan ? -1 : cnt;
+            if (scan) {
+                const uint32_t k = atomicAdd(scanq_n + CTR_GEOQ, 1u);
+                if (k < n) *geo_queue_entry(scanq, n, k) = i;
             }
         }
         __syncwarp();
@@ -914,21 +960,21 @@ cudaError_t launch_density(const DevParams& P, const StepBuffers& b, cudaStream_
             PFS_LAUNCH(k_density_slab, g, b.xp, b.table, b.order, b.rr, b.err);
             break;
         default:
-            if (b.variant == NBR_FLAT)
-                PFS_LAUNCH(k_density_flat, g, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
-                           b.scanq_n, b.err);
-            else
-                PFS_LAUNCH(k_density_list, g, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
-                           b.scanq_n, b.err);
-            if (b.geo_any) {
-                if (b.sr.scenes)
-                    k_density_geo<true><<<geo_grid(k_density_geo<true>, P.n), GEO_WARPS * 32, 0, s>>>(
-                        P, b.sr, b.xp, b.table, b.order, b.bucket, b.brank, b.bcount, b.boffset,
-                        b.nblocks, b.rr, b.nlist, b.ncount, b.scanq, b.scanq_n, b.err);
+            if (!b.all_geo) {
+                if (b.variant == NBR_FLAT)
+                    PFS_LAUNCH(k_density_flat, g, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
+                               b.scanq_n, b.err);
                 else
-                    k_density_geo<false><<<geo_grid(k_density_geo<false>, P.n), GEO_WARPS * 32, 0, s>>>(
-                        P, b.sr, b.xp, b.table, b.order, b.bucket, b.brank, b.bcount, b.boffset,
-                        b.nblocks, b.rr, b.nlist, b.ncount, b.scanq, b.scanq_n, b.err);
+                    PFS_LAUNCH(k_density_list, g, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
+                               b.scanq_n, b.err);
+            }
+            if (b.geo_any) {
+                const cudaError_t e = launch_cells(P, b, Dens32{b.xp}, s);
+                if (e != cudaSuccess) return e;
+                auto k = b.sr.scenes ? k_density_geo<true> : k_density_geo<false>;
+                k<<<geo_grid(k, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, b.table, b.order, b.bcount,
+                                                              b.boffset, b.keys_tmp, b.rr, b.nlist, b.ncount,
+                                                              b.scanq, b.scanq_n, b.err);
             }
     }
     return cudaGetLastError();

@@ -14,6 +14,7 @@
 // reference's predict-then-scatter (predictPositions.comp, scatterPass.comp).
 // The state stays in sort order between substeps, as the reference's
 // ping-pong buffers do.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -61,10 +62,8 @@ k_reorder(DevParams P0, SceneRef sr, const uint32_t* __restrict__ skeys, const u
     const uint32_t n = P0.n;
     if (s == 0) {
         *bcounter = 0u;
-        scanq_n[0] = 0u;  // scan queue
-        scanq_n[1] = 0u;  // grid-search queue
-        scanq_n[2] = 0u;  // grid-search density pass: work counter
-        scanq_n[3] = 0u;  // grid-search force pass: work counter
+#pragma unroll
+        for (int k = 0; k < CTR_WORDS; k++) scanq_n[k] = 0u;
         if (st_counters) {  // staged passes: block list and work counters
             st_counters[ST_CTR_BLOCKS] = 0u;
             st_counters[ST_CTR_DENSITY] = 0u;
@@ -106,12 +105,16 @@ k_reorder(DevParams P0, SceneRef sr, const uint32_t* __restrict__ skeys, const u
 // consecutive block ids and reserves one contiguous range for them, so
 // segments land in about block-id order (row-major in space) and the
 // neighbour passes, which take positions in order, sweep space coherently:
-// a neighbourhood's data is reused from L2 while it is hot.
+// a neighbourhood's data is reused from L2 while it is hot.  With the grid
+// search (clist) the non-empty blocks of 2^vshift consecutive buckets are listed
+// in the same order; a block never spans two thread blocks (256 is a multiple of
+// its size, and a batch's scenes start at multiples of 256).
 __global__ void __launch_bounds__(ELEM_THREADS)
 k_bucket_alloc(uint32_t nblocks, const uint32_t* __restrict__ bcount, uint32_t* __restrict__ boffset,
-               uint32_t* __restrict__ bcounter) {
-    __shared__ uint32_t s_warp[ELEM_THREADS / 32];
-    __shared__ uint32_t s_base;
+               uint32_t* __restrict__ bcounter, uint32_t* __restrict__ clist, uint32_t list_n, uint32_t vshift,
+               const uint32_t* __restrict__ cvshift, uint32_t* __restrict__ nlisted) {
+    __shared__ uint32_t s_warp[ELEM_THREADS / 32], s_incl[ELEM_THREADS], s_live[ELEM_THREADS / 32];
+    __shared__ uint32_t s_base, s_list;
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t c = b < nblocks ? bcount[b] : 0u;
@@ -133,7 +136,32 @@ k_bucket_alloc(uint32_t nblocks, const uint32_t* __restrict__ bcount, uint32_t* 
         s_base = run ? atomicAdd(bcounter, run) : 0u;
     }
     __syncthreads();
-    if (c) boffset[b] = s_base + s_warp[warp] + incl - c;
+    const uint32_t before = s_warp[warp] + incl - c;
+    if (c) boffset[b] = s_base + before;
+    if (!clist) return;
+    const uint32_t vs = cvshift ? cvshift[blockIdx.x] : vshift;
+    if (vs >= 32u) return;  // a table-scan scene's buckets
+    s_incl[threadIdx.x] = before + c;
+    __syncthreads();
+    const uint32_t v = 1u << vs;
+    const bool first = (threadIdx.x & (v - 1u)) == 0u && s_incl[threadIdx.x + v - 1u] > before;
+    const uint32_t live = __ballot_sync(0xffffffffu, first);
+    if (lane == 0) s_live[warp] = __popc(live);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t run = 0;
+        for (int w = 0; w < ELEM_THREADS / 32; w++) {
+            const uint32_t t = s_live[w];
+            s_live[w] = run;
+            run += t;
+        }
+        s_list = run ? atomicAdd(nlisted, run) : 0u;
+    }
+    __syncthreads();
+    if (first) {
+        const uint32_t k = s_list + s_live[warp] + __popc(live & ((1u << lane) - 1u));
+        if (k < list_n) clist[k] = b;
+    }
 }
 
 // Step 3: place each slot in its block's segment.  The block counters are
@@ -238,8 +266,9 @@ cudaError_t launch_reorder(const DevParams& P, const StepBuffers& b, cudaStream_
         const cudaError_t e = launch_bucket_alloc_staged(P, b, s);
         if (e != cudaSuccess) return e;
     } else if (nb > 0) {
-        k_bucket_alloc<<<grid_for(nb, ELEM_THREADS), ELEM_THREADS, 0, s>>>(nb, b.bcount, b.boffset,
-                                                                            b.bcounter);
+        k_bucket_alloc<<<grid_for(nb, ELEM_THREADS), ELEM_THREADS, 0, s>>>(
+            nb, b.bcount, b.boffset, b.bcounter, b.geo_any ? b.clist : nullptr, std::min(nb, P.n),
+            (uint32_t)(P.bsx + P.bsy + P.bsz), b.cvshift, b.scanq_n + CTR_BLOCKS);
     }
     k_bucket_scatter<<<g, ELEM_THREADS, 0, s>>>(P.n, nb, b.bucket, b.brank, b.boffset, b.bcount,
                                                 b.geo_any, b.order, b.err);

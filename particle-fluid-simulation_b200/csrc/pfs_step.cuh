@@ -46,7 +46,14 @@ struct StepBuffers {
     int32_t* nlist;     // list_cap * n (DevParams::list_cap)
     int32_t* ncount;    // n
     uint32_t* scanq;    // n: positions t whose force pass must scan
-    uint32_t* scanq_n;  // 1: entries in scanq
+    uint32_t* scanq_n;  // CTR_WORDS counters, zeroed by the reorder
+    // cell-grouped density pass of the grid search (pfs_cells.cuh): the first
+    // bucket of each non-empty block, log2 of the buckets per block for each 256
+    // buckets (batch; a world's own), and the entries a thread block stages
+    uint32_t* clist;    // min(buckets, n)
+    uint32_t* cvshift;  // (buckets + 255) / 256, null for a world
+    uint32_t cells_entries;
+    uint32_t all_geo;   // every particle uses the grid search
     // batch of scenes: per-slot scene parameters (null for one world) and
     // the spatial-order blocks of all scenes together
     SceneRef sr;
@@ -71,6 +78,18 @@ struct StepBuffers {
     // (bit-exact), 1 fused multiply-adds and hardware reciprocals
     // (PFS_FP32_FAST)
     int32_t fast;
+};
+
+// Counters in StepBuffers::scanq_n.
+enum {
+    CTR_SCANQ = 0,     // scan queue (from the bottom of scanq)
+    CTR_GEOQ = 1,      // grid-search queue of the force pass (from the top)
+    CTR_SLOWWORK = 2,  // one-warp-per-particle density pass: work counter
+    CTR_GEOWORK = 3,   // grid-search force pass: work counter
+    CTR_SLOW = 4,      // particles left to the one-warp-per-particle density pass
+    CTR_CELLS = 5,     // cell-grouped density pass: work counter
+    CTR_BLOCKS = 6,    // non-empty blocks of the grid-search particles
+    CTR_WORDS = 8
 };
 
 // Neighbours a list holds per particle.

@@ -47,10 +47,12 @@ static bool choose_grid_search(uint32_t n, const uint32_t g[3], int search) {
     return slots * 4 <= (uint64_t)n;
 }
 
+static void set_block_counts(DevParams* o);
+
 // Same arithmetic as the oracle's pfso_derive: volume per main.c:349 in
 // double, kernel scales per calculateDensities.comp:110 and
 // applyPressureAndViscosityForce.comp:89,104 in float, PI = 3.14159265359f.
-void derive_params(const pfs_params& p, uint32_t n, DevParams* o, int search) {
+void derive_params(const pfs_params& p, uint32_t n, DevParams* o, int search, double fluid, uint32_t members) {
     const float PI = 3.14159265359f;
     const float h = p.h;
     o->h = h;
@@ -81,8 +83,9 @@ void derive_params(const pfs_params& p, uint32_t n, DevParams* o, int search) {
     o->mask = n > 0 ? n - 1u : 0u;
     o->n = n;
     o->flags = p.flags;
-    // grid of cells over the box and the blocks the spatial order groups them
-    // into: 2x2x2 cells, coarser when the box is large against n
+    // grid of cells over the box and the buckets of the spatial order: 2x2x2
+    // cells, or with the grid search single cells in blocks of about `members`
+    // particles (at most 4x4x4); coarser when the box is large against n
     uint32_t g[3];
     for (int a = 0; a < 3; a++) {
         double cells = std::floor(((double)p.box_max[a] - (double)p.box_min[a]) / (double)h) + 1.0;
@@ -90,18 +93,27 @@ void derive_params(const pfs_params& p, uint32_t n, DevParams* o, int search) {
     }
     o->ngx = g[0]; o->ngy = g[1]; o->ngz = g[2];
     o->geo = choose_grid_search(n, g, search) ? 1u : 0u;
-    const double cap = std::max(4.0 * (double)n, 4096.0);
-    // the grid search reads single cells when the buffers allow it
-    int s = o->geo ? 0 : 1;
-    for (;; s++) {
-        const double nb = (double)((g[0] - 1) >> s) + 1.0;
-        const double blocks = nb * ((double)((g[1] - 1) >> s) + 1.0) * ((double)((g[2] - 1) >> s) + 1.0);
-        if (blocks <= cap || s >= 20) break;
+    o->cshift = o->geo ? 0 : 1;
+    o->bsx = o->bsy = o->bsz = 0;
+    o->blayers = 1;
+    // rounding of a cell coordinate u < 2^10: 2^-23 u at most for the two
+    // operations together, so neighbours in range differ by less than
+    // 1 + 2^-22 u; twice that, and at least the FP16 record's 2^-11
+    const float gmax = (float)std::max(g[0], std::max(g[1], g[2]));
+    o->edge = p.precision == PFS_FP16_CELL ? 1.0f / 1024.0f : gmax * (1.0f / 2097152.0f);
+    if (o->geo) {
+        // a thread block of the density pass takes one block: 104 particles fill
+        // its warps; a small world takes smaller blocks, so that it has a few per SM
+        if (members == 0) members = std::min(std::max(n / (3u * 148u), 24u), 104u);
+        const double want = 1.2 * (double)members / cell_density(*o, p, n, fluid);
+        const int total = want >= 64.0 ? 6 : want >= 2.0 ? (int)std::floor(std::log2(want)) : 0;
+        o->bsx = (total + 2) / 3;
+        o->bsy = (total - o->bsx + 1) / 2;
+        o->bsz = total - o->bsx - o->bsy;
     }
-    o->bshift = s;
-    o->nbx = ((g[0] - 1) >> s) + 1;
-    o->nby = ((g[1] - 1) >> s) + 1;
-    o->nbz = ((g[2] - 1) >> s) + 1;
+    const double cap = o->geo ? std::max(16.0 * (double)n, 65536.0) : std::max(4.0 * (double)n, 4096.0);
+    set_block_counts(o);
+    fit_spatial_blocks(o, (uint32_t)std::min(cap, 4294967295.0));
     o->key_base = 0;
     o->block_base = 0;
     o->list_cap = NLIST_CAP;
@@ -117,7 +129,58 @@ void derive_params(const pfs_params& p, uint32_t n, DevParams* o, int search) {
     }
 }
 
-uint32_t spatial_blocks(const DevParams& P) { return P.nbx * P.nby * P.nbz; }
+// Blocks per axis.
+static void set_block_counts(DevParams* o) {
+    o->nbx = ((o->ngx - 1) >> (o->cshift + o->bsx)) + 1;
+    o->nby = ((o->ngy - 1) >> (o->cshift + o->bsy)) + 1;
+    o->nbz = ((o->ngz - 1) >> (o->cshift + o->bsz)) + 1;
+}
+
+static double bucket_count(const DevParams& P) {
+    return (double)P.nbx * (double)P.nby * (double)P.nbz * (double)(1 << (P.bsx + P.bsy + P.bsz));
+}
+
+uint32_t spatial_blocks(const DevParams& P) { return (uint32_t)bucket_count(P); }
+
+double cell_density(const DevParams& P, const pfs_params& p, uint32_t n, double fluid) {
+    double box = 1.0;
+    for (int a = 0; a < 3; a++) box *= (double)p.box_max[a] - (double)p.box_min[a];
+    if (!(fluid > 0.0)) fluid = box / 4.0;  // unknown: a quarter full
+    const double h = p.h, cells = std::max(1.0, std::min(fluid, box) / (h * h * h));
+    return std::max((double)n / cells, (double)n / ((double)P.ngx * P.ngy * P.ngz));
+}
+
+// As many layers of a block's neighbourhood at a time as CELLS_STAGE entries
+// hold, with an eighth to spare; at least one, of up to CELLS_STAGE_MAX entries.
+uint32_t cells_entries(DevParams* P, double per_cell) {
+    const double layer = 1.125 * ((1 << P->bsx) + 2) * ((1 << P->bsy) + 2) * per_cell;
+    const int layers = (1 << P->bsz) + 2;
+    P->blayers = std::min(std::max((int)((CELLS_STAGE - 64.0) / layer), 1), layers);
+    const double want = std::min(std::max(layer * P->blayers + 64.0, 384.0), (double)CELLS_STAGE_MAX);
+    return ((uint32_t)want + 63u) & ~63u;
+}
+
+double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4) {
+    if (!pos4 || n == 0) return 0.0;
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, pos4) != cudaSuccess)
+        cudaGetLastError();
+    else if (attr.type == cudaMemoryTypeDevice)
+        return 0.0;
+    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    const uint32_t step = std::max(1u, n / 4096u);
+    for (uint32_t i = 0; i < n; i += step)
+        for (int a = 0; a < 3; a++) {
+            const double v = pos4[4 * (size_t)i + a];
+            if (v >= p.box_min[a] && v <= p.box_max[a]) {
+                lo[a] = std::min(lo[a], v);
+                hi[a] = std::max(hi[a], v);
+            }
+        }
+    double vol = 1.0;
+    for (int a = 0; a < 3; a++) vol *= hi[a] >= lo[a] ? std::max(hi[a] - lo[a], (double)p.h) : (double)p.h;
+    return vol;
+}
 
 bool grid_search_allowed(const pfs_params& p, uint32_t n) {
     DevParams d{};
@@ -125,13 +188,15 @@ bool grid_search_allowed(const pfs_params& p, uint32_t n) {
     return d.geo != 0;
 }
 
-// Coarsen the spatial-order blocks until they fit buffers sized for `cap`.
+// Coarsen the spatial order until its buckets fit buffers sized for `cap`: give
+// the blocks (and their padding) up first, then join cells.
 void fit_spatial_blocks(DevParams* o, uint32_t cap) {
-    while (spatial_blocks(*o) > cap && o->bshift < 20) {
-        o->bshift++;
-        o->nbx = ((o->ngx - 1) >> o->bshift) + 1;
-        o->nby = ((o->ngy - 1) >> o->bshift) + 1;
-        o->nbz = ((o->ngz - 1) >> o->bshift) + 1;
+    while (bucket_count(*o) > (double)cap && o->cshift < 20) {
+        if (o->bsx + o->bsy + o->bsz)
+            o->bsx = o->bsy = o->bsz = 0;
+        else
+            o->cshift++;
+        set_block_counts(o);
     }
 }
 
@@ -173,7 +238,7 @@ void* Arena::take(size_t n) {
 size_t world_arena_bytes(uint32_t n, int flags, int precision, uint32_t blocks, uint32_t list_cap,
                          uint32_t staged_blocks) {
     const size_t f4 = (size_t)n * 16, u = (size_t)n * 4;
-    size_t b = 6 * f4 /*x v xs vs xp vp*/ + (size_t)n * 8 /*rr*/ + 5 * u /*keys skeys perm tmp x2*/ +
+    size_t b = u /*clist*/ + 6 * f4 /*x v xs vs xp vp*/ + (size_t)n * 8 /*rr*/ + 5 * u /*keys skeys perm tmp x2*/ +
                sort_scratch_words(n, sort_key_bits(n)) * 4 + (size_t)n * 8 /*table*/ + 256 /*err*/ +
                3 * u /*order bucket brank*/ + 2 * (size_t)blocks * 4 /*bcount boffset*/ + 256 +
                (size_t)(list_cap + 2) * u /*nlist ncount scanq*/ + 256;
@@ -206,6 +271,7 @@ struct pfs_world {
     pfs_stage_times times{};
     bool sorted_valid = false;  // skeys/perm hold a sort result
     uint32_t blocks_cap = 0;    // spatial-order buckets the arena holds
+    double fluid = 0.0;         // volume the initial state's particles fill (fluid_volume)
     int search = -1;            // neighbour search: -1 automatic, 0 table, 1 grid
     // staged shape (pfs_staged.cu): block shape picked from the initial
     // state's density, or unavailable (grid too large for fine buckets)
@@ -321,6 +387,12 @@ int capture_graph(pfs_world* w) {
 
 int set_device(pfs_world* w) { return status_from_cuda(cudaSetDevice(w->device)); }
 
+// The grid search's flags and staging for the world's current parameters.
+void set_cells(pfs_world* w) {
+    w->b.geo_any = w->b.all_geo = w->dp.geo;
+    w->b.cells_entries = cells_entries(&w->dp, cell_density(w->dp, w->params, w->n, w->fluid));
+}
+
 int carve(pfs_world* w) {
     const uint32_t n = w->n;
     Arena& a = w->arena;
@@ -363,15 +435,17 @@ int carve(pfs_world* w) {
     b.btot = (uint32_t*)a.take(((size_t)w->staged_blocks + 1) * 4);
     b.blist = (uint32_t*)a.take(((size_t)w->staged_blocks + 1) * 4);
     b.st_counters = (uint32_t*)a.take(256);
+    b.clist = (uint32_t*)a.take(u);
+    b.cvshift = nullptr;
+    set_cells(w);
     b.fast = w->params.precision == PFS_FP32_FAST ? 1 : 0;
     b.sr = SceneRef{nullptr, nullptr};
     b.nblocks = spatial_blocks(w->dp);
-    b.geo_any = w->dp.geo;
     // the FP16-cell form has one shape, the list shape's
     b.variant = w->params.precision == PFS_FP16_CELL ? (int)NBR_LIST : nbr_variant();
     if (!b.order || !b.bucket || !b.brank || !b.bcount || !b.boffset || !b.bcounter ||
         !b.nlist || !b.ncount || !b.scanq || !b.scanq_n || !b.bseg || !b.btot || !b.blist ||
-        !b.st_counters)
+        !b.st_counters || !b.clist)
         return PFS_ENOMEM;
     b.ids = b.ids_s = nullptr;
     b.color = nullptr;
@@ -564,7 +638,8 @@ int pfs_world_create(const pfs_params* p, uint32_t n, const float* pos4, const f
     w->n = n;
     w->flags = p->flags;
     if (w->flags & PFS_FLAG_IDS) w->flags |= PFS_FLAG_IDS_INTERNAL;
-    derive_params(*p, n, &w->dp);
+    w->fluid = fluid_volume(*p, n, pos4);
+    derive_params(*p, n, &w->dp, -1, w->fluid);
     w->list_cap = list_rows_for(*p, n, pos4);
     w->dp.list_cap = w->list_cap;
     {
@@ -622,11 +697,11 @@ int pfs_world_set_params(pfs_world* w, const pfs_params* p) {
     if ((rc = wait_stream(w, 0))) return rc;
     const bool rekey = p->h != w->params.h || std::memcmp(p->box_min, w->params.box_min, 12) != 0;
     w->params = *p;
-    derive_params(*p, w->n, &w->dp, w->search);
+    derive_params(*p, w->n, &w->dp, w->search, w->fluid);
     w->dp.list_cap = w->list_cap;
     fit_spatial_blocks(&w->dp, w->blocks_cap);
     w->b.nblocks = spatial_blocks(w->dp);
-    w->b.geo_any = w->dp.geo;
+    set_cells(w);
     drop_graph(w);
     if (rekey) {
         cudaError_t e = launch_keys(w->dp, w->b, w->stream);
@@ -1233,7 +1308,7 @@ static int apply_shape(pfs_world* w, int32_t shape, int32_t search) {
     }
     w->b.variant = shape;
     w->search = search;
-    derive_params(w->params, w->n, &w->dp, search);
+    derive_params(w->params, w->n, &w->dp, search, w->fluid);
     w->dp.list_cap = w->list_cap;
     if (shape == NBR_STAGED) {
         const DevParams& c = w->staged_cfg;
@@ -1249,7 +1324,7 @@ static int apply_shape(pfs_world* w, int32_t shape, int32_t search) {
         fit_spatial_blocks(&w->dp, w->blocks_cap);
         w->b.nblocks = spatial_blocks(w->dp);
     }
-    w->b.geo_any = w->dp.geo;
+    set_cells(w);
     drop_graph(w);
     return PFS_OK;
 }
