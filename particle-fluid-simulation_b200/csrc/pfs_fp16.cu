@@ -392,26 +392,30 @@ k_force16(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const float4
     const float2 rri = rr[i];
     const Self16 s = self16(P, rec[i], vp[i], rri);
     Acc16 f = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    auto index = [&](int32_t k) -> int32_t {
-        const int32_t j = k < cnt ? __ldg(nlist + (size_t)k * n + t) : (int32_t)i;
-        if ((uint32_t)j >= n) {
-            atomicOr(err, ERR_TABLE_RANGE);
-            return (int32_t)i;  // self: distance 0, skipped
-        }
-        return j;
+    // four neighbours at a time, their data in flight together, the next four's
+    // indices too; past the end the particle itself (distance 0, skipped)
+    int32_t jn[4];
+    auto indices = [&](int32_t k) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) jn[u] = k + u < cnt ? __ldg(nlist + (size_t)(k + u) * n + t) : (int32_t)i;
     };
-    int32_t jn = index(1);
-    int32_t j = index(0);
-    uint4 r = __ldg(rec + j);
-    float2 rj = __ldg(rr + j);
-    for (int32_t k = 0; k < cnt; k++) {
-        const int32_t jnn = index(k + 2);
-        const uint4 rn = __ldg(rec + jn);
-        const float2 rjn = __ldg(rr + jn);
-        force16_term(P, s, rec_unpack(r), rj, f);
-        r = rn;
-        rj = rjn;
-        jn = jnn;
+    indices(0);
+    for (int32_t k = 0; k < cnt; k += 4) {
+        int32_t j[4] = {jn[0], jn[1], jn[2], jn[3]};
+        indices(k + 4);
+        uint4 r[4];
+        float2 rj[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if ((uint32_t)j[u] >= n) {
+                atomicOr(err, ERR_TABLE_RANGE);
+                j[u] = (int32_t)i;
+            }
+            r[u] = __ldg(rec + j[u]);
+            rj[u] = __ldg(rr + j[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) force16_term(P, s, rec_unpack(r[u]), rj[u], f);
     }
     vout[i] = force16_finish(P, f, vs[i], rri.x);
 }

@@ -287,32 +287,37 @@ k_force_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const flo
     const float2 rri = __ldcs(rr + i);
     const ForceSelf me = force_self(P, __ldcs(xp + i), __ldcs(vp + i), rri);
     ForceAcc f = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    // software pipeline: the index of neighbour k+2 and the data of k+1 are
-    // in flight while neighbour k is evaluated
-    auto index = [&](int32_t k) -> int32_t {
-        const int32_t j = k < cnt ? __ldcs(nlist + (size_t)k * n + t) : (int32_t)i;
-        if ((uint32_t)j >= n) {
-            atomicOr(err, ERR_TABLE_RANGE);
-            return (int32_t)i;  // evaluated as self: d = 0, skipped
-        }
-        return j;
+    // four neighbours at a time, their data in flight together, the next four's
+    // indices too; past the end the particle itself (distance 0, skipped)
+    int32_t jn[4];
+    auto indices = [&](int32_t k) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) jn[u] = k + u < cnt ? __ldcs(nlist + (size_t)(k + u) * n + t) : (int32_t)i;
     };
-    int32_t jn = index(1);
-    int32_t j = index(0);
-    float4 q = __ldg(xp + j), vj = __ldg(vs + j);
-    float2 rj = __ldg(rr + j);
-    for (int32_t k = 0; k < cnt; k++) {
-        const int32_t jnn = index(k + 2);
-        const float4 qn = __ldg(xp + jn), vn = __ldg(vs + jn);
-        const float2 rn = __ldg(rr + jn);
-        if constexpr (FAST)
-            force_term_fast(P, me, make_float4(q.x, q.y, q.z, rj.x), make_float4(vj.x, vj.y, vj.z, rj.y), f);
-        else
-            force_term_pre(P, me, q, rj, vj, f);
-        q = qn;
-        vj = vn;
-        rj = rn;
-        jn = jnn;
+    indices(0);
+    for (int32_t k = 0; k < cnt; k += 4) {
+        int32_t j[4] = {jn[0], jn[1], jn[2], jn[3]};
+        indices(k + 4);
+        float4 q[4], vj[4];
+        float2 rj[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if ((uint32_t)j[u] >= n) {
+                atomicOr(err, ERR_TABLE_RANGE);
+                j[u] = (int32_t)i;
+            }
+            q[u] = __ldg(xp + j[u]);
+            vj[u] = __ldg(vs + j[u]);
+            rj[u] = __ldg(rr + j[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if constexpr (FAST)
+                force_term_fast(P, me, make_float4(q[u].x, q[u].y, q[u].z, rj[u].x),
+                                make_float4(vj[u].x, vj[u].y, vj[u].z, rj[u].y), f);
+            else
+                force_term_pre(P, me, q[u], rj[u], vj[u], f);
+        }
     }
     __stcs(vout + i, force_finish(P, f, __ldcs(vs + i), rri.x));
 }
