@@ -164,6 +164,57 @@ __device__ __forceinline__ void force_term(const DevParams& P, const ForceSelf& 
     force_term_pre(P, me, __ldg(xp + j), __ldg(rr + j), __ldg(vs + j), f);
 }
 
+// a / b given y = RN(1 / b), by Markstein's correction (P. Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990): the
+// residual of RN(a y) is exact in one fused operation, and the corrected quotient
+// is the correctly rounded one, as long as nothing underflows or overflows.
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+    const float q = PFS_MUL(a, y);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+
+// The five quotients of a neighbour's force terms: its direction d / dist, and
+// the pressure and viscosity coefficients c / dj and v / dj (dj >= 0.01).  Two
+// reciprocals serve all five; a third of the pass's instructions were the
+// divisions.  The correction holds while every numerator is zero or in
+// [2^-75, 2^75] and the denominators are in [2^-30, 2^45] (dist is in
+// [1e-7, h]): quotients then stay in [2^-120, 2^105] and residuals above 2^-99.
+// Anything else (piles' densities, coordinates near 2^-52, NaN) is divided.
+// (A zero numerator gives +0 where a division may give -0: the terms are added
+// to sums that start at +0, where the two are the same.)
+struct ForceQuot {
+    float x, y, z, coef, vcoef;
+};
+__device__ __forceinline__ ForceQuot force_quot(const DevParams& P, float d0, float d1, float d2, float dist,
+                                                float dj, float c, float v) {
+    ForceQuot r;
+    const float yd = __frcp_rn(dist), yj = __frcp_rn(dj);
+    r.x = div_by(d0, dist, yd);
+    r.y = div_by(d1, dist, yd);
+    r.z = div_by(d2, dist, yd);
+    r.coef = div_by(c, dj, yj);
+    r.vcoef = div_by(v, dj, yj);
+    // twice the bits less one: the sign drops out and zero becomes the largest
+    auto low = [](float x) { return 2u * __float_as_uint(x) - 1u; };
+    const uint32_t least = min(min(min(low(d0), low(d1)), low(d2)), min(low(c), low(v)));
+    const bool fine = least >= 2u * 0x1a000000u - 1u /* 2^-75 */ && fmaxf(fabsf(c), fabsf(v)) <= 0x1p75f &&
+                      dj <= 0x1p45f && P.h <= 0x1p45f;
+    if (!fine) {
+        r.x = PFS_DIV(d0, dist);
+        r.y = PFS_DIV(d1, dist);
+        r.z = PFS_DIV(d2, dist);
+        r.coef = PFS_DIV(c, dj);
+        r.vcoef = PFS_DIV(v, dj);
+    }
+    return r;
+}
+
+// With kn = 0 (and finite near densities) the near pressure is +-0: its terms
+// leave the sums as they are and are not evaluated.
+__device__ __forceinline__ bool near_vanishes(const DevParams& P, const ForceSelf& me, float nnd) {
+    return P.kn == 0.0f && me.near_pressure == 0.0f && fabsf(nnd) < INFINITY;
+}
+
 __device__ __forceinline__ void force_term_pre(const DevParams& P, const ForceSelf& me,
                                                const float4 q, const float2 rrj, const float4 vj,
                                                ForceAcc& f) {
@@ -172,28 +223,27 @@ __device__ __forceinline__ void force_term_pre(const DevParams& P, const ForceSe
     const float dd = dist2(q, me.sp, d0, d1, d2);
     const float dist = PFS_SQRT(dd);
     if (fabsf(dist) < 1e-7f) return;
-    const float dirx = PFS_DIV(d0, dist), diry = PFS_DIV(d1, dist), dirz = PFS_DIV(d2, dist);
     const float slope = PFS_MUL(PFS_SUB(dist, h), P.slope_scale);
     const float dj = rrj.x;
     // (a + b) / 2 and (a + b) * 0.5 are the same correctly rounded value
     const float shared = PFS_MUL(PFS_ADD(PFS_MUL(PFS_SUB(dj, P.rho0), P.k), me.my_pressure_term), 0.5f);
-    const float coef = PFS_DIV(PFS_MUL(PFS_MUL(shared, slope), m), dj);
-    f.fpx = PFS_ADD(f.fpx, PFS_MUL(coef, dirx));
-    f.fpy = PFS_ADD(f.fpy, PFS_MUL(coef, diry));
-    f.fpz = PFS_ADD(f.fpz, PFS_MUL(coef, dirz));
     const float a = PFS_SUB(h, dist);
     const float a2 = PFS_MUL(a, a);
-    const float vcoef = PFS_DIV(PFS_MUL(m, a2), dj);
-    f.fvx = PFS_ADD(f.fvx, PFS_MUL(vcoef, PFS_SUB(vj.x, me.pv.x)));
-    f.fvy = PFS_ADD(f.fvy, PFS_MUL(vcoef, PFS_SUB(vj.y, me.pv.y)));
-    f.fvz = PFS_ADD(f.fvz, PFS_MUL(vcoef, PFS_SUB(vj.z, me.pv.z)));
+    const ForceQuot r = force_quot(P, d0, d1, d2, dist, dj, PFS_MUL(PFS_MUL(shared, slope), m), PFS_MUL(m, a2));
+    f.fpx = PFS_ADD(f.fpx, PFS_MUL(r.coef, r.x));
+    f.fpy = PFS_ADD(f.fpy, PFS_MUL(r.coef, r.y));
+    f.fpz = PFS_ADD(f.fpz, PFS_MUL(r.coef, r.z));
+    f.fvx = PFS_ADD(f.fvx, PFS_MUL(r.vcoef, PFS_SUB(vj.x, me.pv.x)));
+    f.fvy = PFS_ADD(f.fvy, PFS_MUL(r.vcoef, PFS_SUB(vj.y, me.pv.y)));
+    f.fvz = PFS_ADD(f.fvz, PFS_MUL(r.vcoef, PFS_SUB(vj.z, me.pv.z)));
     const float nnd = rrj.y;
+    if (near_vanishes(P, me, nnd)) return;
     const float shared_near = PFS_MUL(PFS_ADD(me.near_pressure, PFS_MUL(nnd, P.kn)), 0.5f);
     const float nslope = PFS_MUL(a2, P.near_slope_scale);
     const float ncoef = PFS_DIV(PFS_MUL(PFS_MUL(shared_near, nslope), m), nnd);
-    f.fpx = PFS_ADD(f.fpx, PFS_MUL(ncoef, dirx));
-    f.fpy = PFS_ADD(f.fpy, PFS_MUL(ncoef, diry));
-    f.fpz = PFS_ADD(f.fpz, PFS_MUL(ncoef, dirz));
+    f.fpx = PFS_ADD(f.fpx, PFS_MUL(ncoef, r.x));
+    f.fpy = PFS_ADD(f.fpy, PFS_MUL(ncoef, r.y));
+    f.fpz = PFS_ADD(f.fpz, PFS_MUL(ncoef, r.z));
 }
 
 __device__ __forceinline__ float4 force_finish(const DevParams& P, const ForceAcc& f, float4 vi,
