@@ -363,7 +363,7 @@ k_force16(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const float4
           const float2* __restrict__ rr, const int2* __restrict__ table,
           const uint32_t* __restrict__ order, const int32_t* __restrict__ nlist,
           const int32_t* __restrict__ ncount, const uint32_t* __restrict__ scanq,
-          const uint32_t* __restrict__ scanq_n, uint32_t qblocks, float4* __restrict__ vout,
+          const uint32_t* __restrict__ scanq_n, uint32_t qblocks, uint32_t in_order, float4* __restrict__ vout,
           uint32_t* __restrict__ err) {
     const uint32_t n = P0.n;
     if (blockIdx.x < qblocks) {
@@ -379,7 +379,8 @@ k_force16(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const float4
         }
         return;
     }
-    const uint32_t t = list_length_order((blockIdx.x - qblocks) * blockDim.x, n, ncount);
+    const uint32_t tb = (blockIdx.x - qblocks) * blockDim.x;
+    const uint32_t t = in_order ? tb + threadIdx.x : list_length_order(tb, n, ncount);
     if (t >= n) return;
     const int32_t cnt = ncount[t];
     if (cnt < 0) return;
@@ -791,11 +792,11 @@ cudaError_t launch_force_fp16(const DevParams& P, const StepBuffers& b, const Fp
     if (b.sr.scenes)
         k_force16<true><<<qb + g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, f.rec, b.rr, b.table,
                                                        b.order, b.nlist, b.ncount, b.scanq,
-                                                       b.scanq_n, qb, b.v, b.err);
+                                                       b.scanq_n, qb, b.all_geo, b.v, b.err);
     else
         k_force16<false><<<qb + g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, f.rec, b.rr,
                                                         b.table, b.order, b.nlist, b.ncount,
-                                                        b.scanq, b.scanq_n, qb, b.v, b.err);
+                                                        b.scanq, b.scanq_n, qb, b.all_geo, b.v, b.err);
     if (b.geo_any) {
                 if (b.sr.scenes)
             k_force16_geo<true><<<geo16_grid(k_force16_geo<true>, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, f.rec, b.rr,

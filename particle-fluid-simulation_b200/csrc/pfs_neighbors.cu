@@ -256,7 +256,7 @@ k_force_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const flo
              const int2* __restrict__ table, const uint32_t* __restrict__ order,
              const int32_t* __restrict__ nlist, const int32_t* __restrict__ ncount,
              const uint32_t* __restrict__ scanq, const uint32_t* __restrict__ scanq_n,
-             uint32_t qblocks, float4* __restrict__ vout,
+             uint32_t qblocks, uint32_t in_order, float4* __restrict__ vout,
              uint32_t* __restrict__ err) {
     const uint32_t n = P0.n;
     if (blockIdx.x < qblocks) {
@@ -272,7 +272,8 @@ k_force_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const flo
         }
         return;
     }
-    const uint32_t t = list_length_order((blockIdx.x - qblocks) * blockDim.x, n, ncount);
+    const uint32_t tb = (blockIdx.x - qblocks) * blockDim.x;
+    const uint32_t t = in_order ? tb + threadIdx.x : list_length_order(tb, n, ncount);
     if (t >= n) return;
     const int32_t cnt = ncount[t];
     if (cnt < 0) return;  // in the queue
@@ -1004,7 +1005,7 @@ cudaError_t launch_force(const DevParams& P, const StepBuffers& b, cudaStream_t 
             auto kf = b.sr.scenes ? (b.fast ? k_force_list<true, true> : k_force_list<true, false>)
                                   : (b.fast ? k_force_list<false, true> : k_force_list<false, false>);
             kf<<<qb + g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, b.rr, b.table, b.order, b.nlist,
-                                              b.ncount, b.scanq, b.scanq_n, qb, b.v, b.err);
+                                              b.ncount, b.scanq, b.scanq_n, qb, b.all_geo, b.v, b.err);
             if (b.geo_any) {
                 if (b.sr.scenes)
                     k_force_geo<true><<<geo_grid(k_force_geo<true>, P.n), GEO_WARPS * 32, 0, s>>>(

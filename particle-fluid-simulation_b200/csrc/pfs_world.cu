@@ -615,7 +615,7 @@ static uint32_t list_rows_for(const pfs_params& p, uint32_t n, const float* pos4
     double vol = 1.0;
     for (int a = 0; a < 3; a++) vol *= std::max(hi[a] - lo[a], (double)p.h);
     const double h = p.h;
-    const double nb = 2.0 * (double)n / vol * (4.0 / 3.0) * 3.14159265358979 * h * h * h;
+    const double nb = 8.0 * (double)n / vol * (4.0 / 3.0) * 3.14159265358979 * h * h * h;
     if (!(nb > NLIST_CAP)) return NLIST_CAP;
     if (nb >= NLIST_CAP_MAX) return NLIST_CAP_MAX;
     return std::min<uint32_t>(((uint32_t)nb + 15u) & ~15u, NLIST_CAP_MAX);
