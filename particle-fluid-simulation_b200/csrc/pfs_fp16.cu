@@ -424,13 +424,13 @@ k_force16(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const float4
 // ---- grid search (pfs_geo.cuh): one warp per particle ------------------------
 
 constexpr int GEO16_DCAP = 512;
-constexpr int GEO16_FCAP = 256;
+constexpr int GEO16_FCAP = 256;   // of them with their force increments
+constexpr int GEO16_JCAP = 1024;  // in the force pass, by slot number alone
 
 // Density pass of the grid-search particles the cell-grouped pass leaves
-// (slowq): same sums in the same order, same list and queue decisions.  Nine
-// blocks per SM, as k_density_geo.
+// (slowq): same sums in the same order, same list and queue decisions.
 template <bool BATCH>
-__global__ void __launch_bounds__(GEO_WARPS * 32, 9)
+__global__ void __launch_bounds__(GEO_WARPS * 32, 6)
 k_density16_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const uint4* __restrict__ rec,
                 const int2* __restrict__ table, const uint32_t* __restrict__ order,
                 const uint32_t* __restrict__ bcount, const uint32_t* __restrict__ boffset,
@@ -621,7 +621,7 @@ k_force16_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const fl
               const uint32_t* __restrict__ boffset, const uint32_t* __restrict__ scanq,
               const uint32_t* __restrict__ scanq_n, float4* __restrict__ vout,
               uint32_t* __restrict__ err) {
-    __shared__ int32_t s_j[GEO_WARPS][GEO16_FCAP];
+    __shared__ int32_t s_j[GEO_WARPS][GEO16_JCAP];
     __shared__ float s_inc[GEO_WARPS][6][GEO16_FCAP];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t full = 0xffffffffu;
@@ -656,32 +656,48 @@ k_force16_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const fl
                 se = make_int2(-1, -1);
             }
         }
-        const int m = warp_gather(P, sp.x, sp.y, sp.z, bcount, boffset, order, sj, GEO16_FCAP, err,
+        const int m = warp_gather(P, sp.x, sp.y, sp.z, bcount, boffset, order, sj, GEO16_JCAP, err,
                                   [&](int32_t j) {
                                       if (j == (int32_t)i) return false;
                                       float ex, ey, ez;
                                       return rec_q2(rec_unpack(__ldg(rec + j)), s.me, ex, ey, ez) < 1.0f;
                                   });
         float acc = 0.0f;  // lanes 0..5: fpx fpy fpz fvx fvy fvz
-        if (m <= GEO16_FCAP) {
+        if (m <= GEO16_JCAP) {
             warp_sort(sj, m);
-            for (int k = lane; k < m; k += 32) {
-                const int32_t j = sj[k];
-                float v[6];
-                force16_incr(P, s, rec_unpack(__ldg(rec + j)), __ldg(rr + j), v);
-#pragma unroll
-                for (int c = 0; c < 6; c++) inc[c][k] = v[c];
-            }
             int lo = 0, hi = 0;
             if (se.x != -1) {
                 lo = geo_lower(sj, m, se.x);
                 hi = geo_lower(sj, m, se.y);
             }
-            __syncwarp();
+            // increments of sj[k0 .. k1) into columns 0 ..
+            auto fill = [&](int k0, int k1) {
+                for (int k = k0 + lane; k < k1; k += 32) {
+                    const int32_t j = sj[k];
+                    float v[6];
+                    force16_incr(P, s, rec_unpack(__ldg(rec + j)), __ldg(rr + j), v);
+#pragma unroll
+                    for (int c = 0; c < 6; c++) inc[c][k - k0] = v[c];
+                }
+                __syncwarp();
+            };
+            // all at once where they fit, else run by run
+            const bool once = m <= GEO16_FCAP;
+            if (once) fill(0, m);
             for (int d = 0; d < 27; d++) {
                 const int l = __shfl_sync(full, lo, d), u = __shfl_sync(full, hi, d);
-                if (lane < 6)
-                    for (int k = l; k < u; k++) acc += inc[lane][k];
+                if (once) {
+                    if (lane < 6)
+                        for (int k = l; k < u; k++) acc += inc[lane][k];
+                    continue;
+                }
+                for (int base = l; base < u; base += GEO16_FCAP) {
+                    const int e = min(base + GEO16_FCAP, u);
+                    fill(base, e);
+                    if (lane < 6)
+                        for (int k = 0; k < e - base; k++) acc += inc[lane][k];
+                    __syncwarp();
+                }
             }
         } else {
             for (int d = 0; d < 27; d++) {
@@ -788,24 +804,14 @@ cudaError_t launch_force_fp16(const DevParams& P, const StepBuffers& b, const Fp
     const unsigned g = grid_for(P.n, NBR_THREADS);
     // one queue thread per possible entry: dense scenes can send most
     // particles to the queue (lists overflow); surplus queue blocks exit at once
-    const unsigned qb = g;
-    if (b.sr.scenes)
-        k_force16<true><<<qb + g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, f.rec, b.rr, b.table,
-                                                       b.order, b.nlist, b.ncount, b.scanq,
-                                                       b.scanq_n, qb, b.all_geo, b.v, b.err);
-    else
-        k_force16<false><<<qb + g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, f.rec, b.rr,
-                                                        b.table, b.order, b.nlist, b.ncount,
-                                                        b.scanq, b.scanq_n, qb, b.all_geo, b.v, b.err);
+    const unsigned qb = b.all_geo ? 0u : g;
+    auto k = b.sr.scenes ? k_force16<true> : k_force16<false>;
+    k<<<qb + g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, f.rec, b.rr, b.table, b.order, b.nlist, b.ncount,
+                                     b.scanq, b.scanq_n, qb, b.all_geo, b.v, b.err);
     if (b.geo_any) {
-                if (b.sr.scenes)
-            k_force16_geo<true><<<geo16_grid(k_force16_geo<true>, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, f.rec, b.rr,
-                                                              b.table, b.order, b.bcount, b.boffset,
-                                                              b.scanq, b.scanq_n, b.v, b.err);
-        else
-            k_force16_geo<false><<<geo16_grid(k_force16_geo<false>, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, f.rec, b.rr,
-                                                               b.table, b.order, b.bcount, b.boffset,
-                                                               b.scanq, b.scanq_n, b.v, b.err);
+        auto kg = b.sr.scenes ? k_force16_geo<true> : k_force16_geo<false>;
+        kg<<<geo16_grid(kg, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, f.rec, b.rr, b.table, b.order,
+                                                          b.bcount, b.boffset, b.scanq, b.scanq_n, b.v, b.err);
     }
     return cudaGetLastError();
 }

@@ -96,35 +96,45 @@ __device__ __forceinline__ int warp_gather(const DevParams& P, float x, float y,
             if (lane >= s) incl += t;
         }
         const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        for (uint32_t base = 0; base < total; base += 32) {
-            const uint32_t t = base + (uint32_t)lane;
-            // block of candidate t: the first lane whose inclusive count exceeds t
-            int lo = 0, hi = 31;
+        // 128 candidates a round, their loads in flight together (a queue holds few
+        // particles, so a warp's own latency is what the pass takes)
+        for (uint32_t base = 0; base < total; base += 128) {
+            int32_t j[4];
+            bool in[4];
 #pragma unroll
-            for (int s = 0; s < 5; s++) {
-                const int mid = (lo + hi) >> 1;
-                const uint32_t v = __shfl_sync(0xffffffffu, incl, mid);
-                if (v <= t)
-                    lo = mid + 1;
-                else
-                    hi = mid;
+            for (int u = 0; u < 4; u++) {
+                const uint32_t t = base + 32u * u + (uint32_t)lane;
+                // block of candidate t: the first lane whose inclusive count exceeds t
+                int lo = 0, hi = 31;
+#pragma unroll
+                for (int s = 0; s < 5; s++) {
+                    const int mid = (lo + hi) >> 1;
+                    const uint32_t v = __shfl_sync(0xffffffffu, incl, mid);
+                    if (v <= t)
+                        lo = mid + 1;
+                    else
+                        hi = mid;
+                }
+                const uint32_t bincl = __shfl_sync(0xffffffffu, incl, lo);
+                const uint32_t bc = __shfl_sync(0xffffffffu, c, lo);
+                const uint32_t bo = __shfl_sync(0xffffffffu, o, lo);
+                j[u] = t < total ? (int32_t)__ldg(order + bo + (t - (bincl - bc))) : -1;
             }
-            const uint32_t bincl = __shfl_sync(0xffffffffu, incl, lo);
-            const uint32_t bc = __shfl_sync(0xffffffffu, c, lo);
-            const uint32_t bo = __shfl_sync(0xffffffffu, o, lo);
-            bool in = false;
-            int32_t j = 0;
-            if (t < total) {
-                j = (int32_t)__ldg(order + bo + (t - (bincl - bc)));
-                if ((uint32_t)j >= n)
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (j[u] >= 0 && (uint32_t)j[u] >= n) {
                     atomicOr(err, ERR_PERM_RANGE);
-                else
-                    in = test(j);
+                    j[u] = -1;
+                }
+                in[u] = j[u] >= 0 && test(j[u]);
             }
-            const uint32_t mask = __ballot_sync(0xffffffffu, in);
-            const int pos = m + __popc(mask & ((1u << lane) - 1u));
-            if (in && pos < cap) s_j[pos] = j;
-            m += __popc(mask);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint32_t mask = __ballot_sync(0xffffffffu, in[u]);
+                const int pos = m + __popc(mask & ((1u << lane) - 1u));
+                if (in[u] && pos < cap) s_j[pos] = j[u];
+                m += __popc(mask);
+            }
         }
     }
     __syncwarp();

@@ -562,7 +562,8 @@ struct Dens32 {
 // In-range candidates a warp holds per particle (beyond them it walks the
 // table ranges instead; same results).
 constexpr int GEO_DCAP = 512;
-constexpr int GEO_FCAP = 256;
+constexpr int GEO_FCAP = 192;   // of them with their force increments
+constexpr int GEO_JCAP = 1024;  // in the force pass, by slot number alone
 constexpr int FORCE_INCS = 9;
 
 // force_term_pre's per-neighbour increments, in its operation order:
@@ -614,11 +615,9 @@ __device__ __forceinline__ float force_chain_add(float acc, int lane, const floa
 
 // Density pass of the grid-search particles the cell-grouped pass leaves (slowq,
 // positions in the processing order).  Same sums, list and queue decisions as
-// k_density_list; particles it cannot list go to the grid-search queue.  Nine blocks of 24 KB fill an SM's shared memory; the
-// register cap of 56 per thread lets the batch form (per-scene parameters)
-// keep all nine resident as well.
+// k_density_list; particles it cannot list go to the grid-search queue.
 template <bool BATCH>
-__global__ void __launch_bounds__(GEO_WARPS * 32, 9)
+__global__ void __launch_bounds__(GEO_WARPS * 32, 6)
 k_density_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const int2* __restrict__ table,
               const uint32_t* __restrict__ order, const uint32_t* __restrict__ bcount,
               const uint32_t* __restrict__ boffset, const uint32_t* __restrict__ slowq,
@@ -813,7 +812,7 @@ k_force_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const floa
             const uint32_t* __restrict__ bcount, const uint32_t* __restrict__ boffset,
             const uint32_t* __restrict__ scanq, uint32_t* __restrict__ scanq_n,
             float4* __restrict__ vout, uint32_t* __restrict__ err) {
-    __shared__ int32_t s_j[GEO_WARPS][GEO_FCAP];
+    __shared__ int32_t s_j[GEO_WARPS][GEO_JCAP];
     __shared__ float s_inc[GEO_WARPS][FORCE_INCS][GEO_FCAP];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t full = 0xffffffffu;
@@ -844,32 +843,48 @@ k_force_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const floa
                 se = make_int2(-1, -1);
             }
         }
-        const int m = warp_gather(P, me.sp.x, me.sp.y, me.sp.z, bcount, boffset, order, sj, GEO_FCAP,
+        const int m = warp_gather(P, me.sp.x, me.sp.y, me.sp.z, bcount, boffset, order, sj, GEO_JCAP,
                                   err, [&](int32_t j) {
                                       if (j == (int32_t)i) return false;
                                       float d0, d1, d2;
                                       return dist2(__ldg(xp + j), me.sp, d0, d1, d2) < P.skip_d2;
                                   });
         float acc = 0.0f;  // lanes 0..5: fpx fpy fpz fvx fvy fvz
-        if (m <= GEO_FCAP) {
+        if (m <= GEO_JCAP) {
             warp_sort(sj, m);
-            for (int k = lane; k < m; k += 32) {
-                const int32_t j = sj[k];
-                float v[FORCE_INCS];
-                force_incr(P, me, __ldg(xp + j), __ldg(rr + j), __ldg(vs + j), v);
-#pragma unroll
-                for (int c = 0; c < FORCE_INCS; c++) inc[c][k] = v[c];
-            }
             int lo = 0, hi = 0;
             if (se.x != -1) {
                 lo = geo_lower(sj, m, se.x);
                 hi = geo_lower(sj, m, se.y);
             }
-            __syncwarp();
+            // increments of sj[k0 .. k1) into columns 0 ..
+            auto fill = [&](int k0, int k1) {
+                for (int k = k0 + lane; k < k1; k += 32) {
+                    const int32_t j = sj[k];
+                    float v[FORCE_INCS];
+                    force_incr(P, me, __ldg(xp + j), __ldg(rr + j), __ldg(vs + j), v);
+#pragma unroll
+                    for (int c = 0; c < FORCE_INCS; c++) inc[c][k - k0] = v[c];
+                }
+                __syncwarp();
+            };
+            // all at once where they fit, else run by run
+            const bool once = m <= GEO_FCAP;
+            if (once) fill(0, m);
             for (int d = 0; d < 27; d++) {
                 const int l = __shfl_sync(full, lo, d), u = __shfl_sync(full, hi, d);
-                if (lane < 6)
-                    for (int k = l; k < u; k++) acc = force_chain_add(acc, lane, inc, k);
+                if (once) {
+                    if (lane < 6)
+                        for (int k = l; k < u; k++) acc = force_chain_add(acc, lane, inc, k);
+                    continue;
+                }
+                for (int base = l; base < u; base += GEO_FCAP) {
+                    const int e = min(base + GEO_FCAP, u);
+                    fill(base, e);
+                    if (lane < 6)
+                        for (int k = 0; k < e - base; k++) acc = force_chain_add(acc, lane, inc, k);
+                    __syncwarp();
+                }
             }
         } else {
             for (int d = 0; d < 27; d++) {
@@ -1000,21 +1015,17 @@ cudaError_t launch_force(const DevParams& P, const StepBuffers& b, cudaStream_t 
             // one queue thread per possible entry: dense scenes can send most
             // particles to the queue (lists overflow), sparse ones very few;
             // surplus queue blocks exit at once
-            const unsigned qb = g;
+            // (the grid search has a queue of its own)
+            const unsigned qb = b.all_geo ? 0u : g;
             // the fast form sums the listed terms with fused arithmetic
             auto kf = b.sr.scenes ? (b.fast ? k_force_list<true, true> : k_force_list<true, false>)
                                   : (b.fast ? k_force_list<false, true> : k_force_list<false, false>);
             kf<<<qb + g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, b.rr, b.table, b.order, b.nlist,
                                               b.ncount, b.scanq, b.scanq_n, qb, b.all_geo, b.v, b.err);
             if (b.geo_any) {
-                if (b.sr.scenes)
-                    k_force_geo<true><<<geo_grid(k_force_geo<true>, P.n), GEO_WARPS * 32, 0, s>>>(
-                        P, b.sr, b.xp, b.vp, b.vs, b.rr, b.table, b.order, b.bcount, b.boffset,
-                        b.scanq, b.scanq_n, b.v, b.err);
-                else
-                    k_force_geo<false><<<geo_grid(k_force_geo<false>, P.n), GEO_WARPS * 32, 0, s>>>(
-                        P, b.sr, b.xp, b.vp, b.vs, b.rr, b.table, b.order, b.bcount, b.boffset,
-                        b.scanq, b.scanq_n, b.v, b.err);
+                auto k = b.sr.scenes ? k_force_geo<true> : k_force_geo<false>;
+                k<<<geo_grid(k, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, b.rr, b.table, b.order,
+                                                              b.bcount, b.boffset, b.scanq, b.scanq_n, b.v, b.err);
             }
         }
     }
