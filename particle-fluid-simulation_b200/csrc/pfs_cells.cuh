@@ -123,7 +123,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 
 // Exclusive scan of v[0, R) in place, R <= 4 * CELLS_THREADS; v[R] and the return
 // value: the total.
-__device__ __forceinline__ uint32_t cells_scan(CellsShared& S, uint32_t* v, uint32_t R) {
+__device__ __forceinline__ uint32_t cells_scan(uint32_t* warp_sum, uint32_t* v, uint32_t R) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t k = 4u * tid;
     uint32_t x[4], own = 0;
@@ -138,13 +138,13 @@ __device__ __forceinline__ uint32_t cells_scan(CellsShared& S, uint32_t* v, uint
         const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += t;
     }
-    if (lane == 31) S.warp_sum[warp] = incl;
+    if (lane == 31) warp_sum[warp] = incl;
     __syncthreads();
     uint32_t base = incl - own, total = 0;
 #pragma unroll
     for (int w = 0; w < CELLS_WARPS; w++) {
-        base += w < warp ? S.warp_sum[w] : 0u;
-        total += S.warp_sum[w];
+        base += w < warp ? warp_sum[w] : 0u;
+        total += warp_sum[w];
     }
 #pragma unroll
     for (int u = 0; u < 4; u++) {
@@ -221,7 +221,7 @@ __device__ __forceinline__ bool cells_build(const DevParams& P, const F& form, C
         }
     }
     __syncthreads();
-    const uint32_t C = cells_scan(S, B.chunk, R);
+    const uint32_t C = cells_scan(S.warp_sum, B.chunk, R);
     // a pile: the neighbourhood has at most six layers, so far more candidates
     // than eight stages hold do not fit; they are not worth reading
     if (C << gs > 8u * E + (R << gs)) return false;
@@ -275,7 +275,7 @@ __device__ __forceinline__ bool cells_build(const DevParams& P, const F& form, C
     if (total > E) return false;
     for (int k = tid; k < CELLS_HASH; k += CELLS_THREADS) S.off[k] = B.cnt[k];
     __syncthreads();
-    cells_scan(S, S.off, CELLS_HASH);
+    cells_scan(S.warp_sum, S.off, CELLS_HASH);
     for (uint32_t k = tid; k < total; k += CELLS_THREADS) {
         const uint32_t hk = zb[k], p = S.off[hk] + atomicSub(&B.cnt[hk], 1u) - 1u;
         sj[p] = zj[k];

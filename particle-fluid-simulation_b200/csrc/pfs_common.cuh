@@ -128,6 +128,14 @@ __device__ __forceinline__ uint32_t spatial_bucket(const DevParams& P, float x, 
     return (blk << (P.sbx + P.sby + P.sbz)) | lx | (ly << P.sbx) | (lz << (P.sbx + P.sby));
 }
 
+// Packed positions of the density map's cell-grouped form: per axis the cell
+// coordinate in steps of 1 / CELLS_CODE_STEPS cell, modulo 512, in a 9-bit field
+// below a guard bit that is set.  Rounding of the coordinate on grids of up to
+// CELLS_MAX_GRID cells per axis (2^-23 of it, twice) stays below one step.
+constexpr int CELLS_CODE_STEPS = 8;
+constexpr uint32_t CELLS_GUARD = (1u << 9) | (1u << 19) | (1u << 29);
+constexpr uint32_t CELLS_MAX_GRID = 1u << 16;
+
 // Entries the cell-grouped density pass stages at a time: 17 KB, so that several
 // thread blocks share an SM; more only where one layer of one cell needs it.
 constexpr uint32_t CELLS_STAGE = 1088;

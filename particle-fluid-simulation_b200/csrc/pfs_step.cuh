@@ -149,9 +149,9 @@ cudaError_t launch_integrate(const DevParams& P, const StepBuffers& b, cudaStrea
 // Density map of the state x (in the order of the last sort, skeys) over an
 // image of image[] voxels of cell_size, with the shader's bounds rule at
 // bound[], into out on the device (the reference's updateDensityMap.comp).
-cudaError_t launch_density_map(const DevParams& P, const StepBuffers& b, float cell_size,
-                               const int32_t image[3], const int32_t bound[3], float* out,
-                               cudaStream_t s);
+// per_cell: particles per cell where the fluid is (sizes the work, not the result).
+cudaError_t launch_density_map(const DevParams& P, const StepBuffers& b, float cell_size, double per_cell,
+                               const int32_t image[3], const int32_t bound[3], float* out, cudaStream_t s);
 
 // Volumetric rendering (pfs_render.cu): light volume of ldims voxels of
 // light_step marched toward sun over the density map dmap (ddims), and the

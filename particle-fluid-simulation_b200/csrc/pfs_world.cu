@@ -937,6 +937,9 @@ static int density_map_extent(const pfs_params& p, float cell_size, int32_t imag
     return voxels > (1ull << 31) ? PFS_ERANGE : PFS_OK;
 }
 
+// Particles per cell where the fluid is, for the density map.
+static double map_density(const pfs_world* w) { return cell_density(w->dp, w->params, w->n, w->fluid); }
+
 int pfs_world_density_map_dims(const pfs_world* w, float cell_size, uint32_t dims[3]) {
     if (!w || !dims) return PFS_EINVAL;
     int32_t img[3], bnd[3];
@@ -1032,7 +1035,7 @@ int pfs_world_render_volumetric(pfs_world* w, const pfs_volume_view* v, uint32_t
         cam[6 + a] = v->right[a];
         cam[9 + a] = v->up[a];
     }
-    cudaError_t e = nd ? launch_density_map(w->dp, w->b, v->density_cell_size, img, bnd, w->map_buf, w->stream)
+    cudaError_t e = nd ? launch_density_map(w->dp, w->b, v->density_cell_size, map_density(w), img, bnd, w->map_buf, w->stream)
                        : cudaSuccess;
     if (e == cudaSuccess && nl)
         e = launch_light_volume(w->dp, w->map_buf, img, v->light_step_size, v->dir_to_sun, ld, lvol,
@@ -1083,7 +1086,7 @@ int pfs_world_render_refractive(pfs_world* w, const pfs_volume_view* v, const pf
         cam[6 + a] = v->right[a];
         cam[9 + a] = v->up[a];
     }
-    cudaError_t e = launch_density_map(w->dp, w->b, v->density_cell_size, img, bnd, w->map_buf, w->stream);
+    cudaError_t e = launch_density_map(w->dp, w->b, v->density_cell_size, map_density(w), img, bnd, w->map_buf, w->stream);
     if (e == cudaSuccess)
         e = launch_refractive(w->dp, w->map_buf, img, cam, half_h, half_w, v->step_size, v->light_step_size,
                               v->extinction, r->num_refractions, r->surface_density_threshold,
@@ -1195,7 +1198,7 @@ int pfs_world_density_map(pfs_world* w, float cell_size, float* out) {
         }
         dst = w->map_buf;
     }
-    cudaError_t e = launch_density_map(w->dp, w->b, cell_size, img, bnd, dst, w->stream);
+    cudaError_t e = launch_density_map(w->dp, w->b, cell_size, map_density(w), img, bnd, dst, w->stream);
     if (e == cudaSuccess && !on_device)
         e = cudaMemcpyAsync(out, dst, voxels * sizeof(float), cudaMemcpyDeviceToHost, w->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(w->stream);
