@@ -110,6 +110,7 @@ struct ViewArgs {
     float3 pos, fwd, right, up;
     float half_h, half_w, step;
     float3 ext;  // normalize(extinctionCoefficients)
+    bool skip_empty;  // coefficients positive, densities finite: no transmittance is Inf or NaN
 };
 
 __device__ __forceinline__ float clamp01(float w) {
@@ -147,6 +148,10 @@ k_volumetric(DevParams P, const float* __restrict__ dmap, int3 dd, const float* 
             const float w1 = clamp01(PFS_DIV(PFS_SUB(PFS_ADD(V.pos.y, PFS_MUL(t, d.y)), P.miny), sy));
             const float w2 = clamp01(PFS_DIV(PFS_SUB(PFS_ADD(V.pos.z, PFS_MUL(t, d.z)), P.minz), sz));
             const float dens = PFS_MUL(tex3d(dmap, dd, w0, w1, w2), 0.05f);
+            // an empty sample leaves the light and the optical depth as they are (its
+            // terms are +0), and most of a box is empty: the light sample and the six
+            // exponentials go (300,000-particle scene, 1280 x 720: 0.29 to 0.16 ms)
+            if (V.skip_empty && dens == 0.0f) continue;
             view = PFS_ADD(view, PFS_MUL(dens, V.step));
             const float sun = tex3d(lvol, ld, w0, w1, w2);
             float in[3], vt[3];
@@ -434,6 +439,9 @@ cudaError_t launch_volumetric(const DevParams& P, const float* dmap, const int32
     V.half_w = half_w;
     V.step = step;
     V.ext = make_float3(ext[0], ext[1], ext[2]);
+    // a density is at most 27 n m h^2 / volume, a march's sum far less than 1e6 of them
+    V.skip_empty = ext[0] > 0.0f && ext[1] > 0.0f && ext[2] > 0.0f &&
+                   27.0 * P.n * fabs((double)P.m) * P.h * P.h < 1e30 * fabs((double)P.volume);
     k_volumetric<<<(unsigned)((n + RENDER_THREADS - 1) / RENDER_THREADS), RENDER_THREADS, 0, s>>>(
         P, dmap, make_int3(ddims[0], ddims[1], ddims[2]), lvol, make_int3(ldims[0], ldims[1], ldims[2]),
         V, width, height, reinterpret_cast<float4*>(rgba));
