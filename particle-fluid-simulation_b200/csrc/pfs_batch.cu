@@ -295,6 +295,7 @@ int pfs_batch_create(uint32_t max_particles, uint32_t max_scenes, int32_t precis
     B->v0 = (float4*)a.take(f4);
     b.sr = SceneRef{B->d_scenes, B->d_sid};
     b.nblocks = 0;
+    b.fp16 = B->precision == PFS_FP16_CELL ? 1u : 0u;
     b.variant = B->precision == PFS_FP16_CELL ? (int)NBR_LIST : nbr_variant();
     bool ok = b.x && b.v && b.xs && b.vs && b.xp && b.vp && b.rr && b.keys && b.skeys && b.perm &&
               b.keys_tmp && b.vals_tmp && b.sort_scratch && b.table && b.err && b.order &&
@@ -626,7 +627,7 @@ int pfs_batch_info_get(pfs_batch* B, pfs_batch_info* out) {
     out->device_bytes = B->arena.bytes;
     bool geo = false;
     for (const Scene& s : B->scenes) geo = geo || s.dp.geo != 0;
-    out->launches_per_substep = substep_launches(B->n_total ? B->n_total : 1, geo);
+    out->launches_per_substep = substep_launches(B->n_total ? B->n_total : 1, geo, false);
     return PFS_OK;
 }
 

@@ -21,6 +21,7 @@
 #include "pfs_fp16.cuh"
 #include "pfs_geo.cuh"
 #include "pfs_record.cuh"
+#include "pfs_small.cuh"
 #include "pfs_step.cuh"
 
 namespace pfs {
@@ -220,6 +221,7 @@ struct Dens16 {
         unpack2(fma2(ex, ex, fma2(ey, ey, mul2(ez, ez))), a, b);
     }
     __device__ __forceinline__ bool in_reach(float q2, float) const { return q2 < 1.0f; }
+    __device__ __forceinline__ bool in_table_reach(float q2, float) const { return q2 < 1.0f; }
     __device__ __forceinline__ void terms(const DevParams&, float q2, float& a2, float& a3) const {
         dens16_terms(q2, a2, a3);
     }
@@ -781,6 +783,7 @@ cudaError_t launch_reorder_fp16(const DevParams& P, const StepBuffers& b, const 
 cudaError_t launch_density_fp16(const DevParams& P, const StepBuffers& b, const Fp16Buffers& f,
                                 cudaStream_t s) {
     if (P.n == 0) return cudaSuccess;
+    if (small_world(P, b)) return launch_density_small(P, b, Dens16{f.rec}, s);
     const unsigned g = grid_for(P.n, NBR_THREADS);
     if (!b.all_geo) {
         auto k = b.sr.scenes ? k_density16_flat<true> : k_density16_flat<false>;

@@ -44,6 +44,7 @@
 #include "pfs_flat.cuh"
 #include "pfs_geo.cuh"
 #include "pfs_nbr.cuh"
+#include "pfs_small.cuh"
 #include "pfs_staged.cuh"
 #include "pfs_step.cuh"
 
@@ -537,6 +538,8 @@ struct Dens32 {
         b = PFS_ADD(PFS_ADD(bx, by), bz);
     }
     __device__ __forceinline__ bool in_reach(float dd, float skip) const { return dd < skip; }
+    // with the table scan a NaN distance takes part (pfs::in_reach)
+    __device__ __forceinline__ bool in_table_reach(float dd, float skip) const { return pfs::in_reach(dd, skip); }
     // density_term's increments; adding them in order gives its sums
     __device__ __forceinline__ void terms(const DevParams& P, float dd, float& t, float& tn) const {
         const float a = PFS_SUB(P.h, PFS_SQRT(dd));
@@ -582,27 +585,27 @@ __device__ __forceinline__ void force_incr(const DevParams& P, const ForceSelf& 
         for (int c = 0; c < FORCE_INCS; c++) inc[c] = 0.0f;
         return;
     }
-    const float dirx = PFS_DIV(d0, dist), diry = PFS_DIV(d1, dist), dirz = PFS_DIV(d2, dist);
     const float slope = PFS_MUL(PFS_SUB(dist, h), P.slope_scale);
     const float dj = rrj.x;
     const float shared = PFS_MUL(PFS_ADD(PFS_MUL(PFS_SUB(dj, P.rho0), P.k), me.my_pressure_term), 0.5f);
-    const float coef = PFS_DIV(PFS_MUL(PFS_MUL(shared, slope), m), dj);
-    inc[0] = PFS_MUL(coef, dirx);
-    inc[1] = PFS_MUL(coef, diry);
-    inc[2] = PFS_MUL(coef, dirz);
     const float a = PFS_SUB(h, dist);
     const float a2 = PFS_MUL(a, a);
-    const float vcoef = PFS_DIV(PFS_MUL(m, a2), dj);
-    inc[3] = PFS_MUL(vcoef, PFS_SUB(vj.x, me.pv.x));
-    inc[4] = PFS_MUL(vcoef, PFS_SUB(vj.y, me.pv.y));
-    inc[5] = PFS_MUL(vcoef, PFS_SUB(vj.z, me.pv.z));
+    const ForceQuot r = force_quot(P, d0, d1, d2, dist, dj, PFS_MUL(PFS_MUL(shared, slope), m), PFS_MUL(m, a2));
+    inc[0] = PFS_MUL(r.coef, r.x);
+    inc[1] = PFS_MUL(r.coef, r.y);
+    inc[2] = PFS_MUL(r.coef, r.z);
+    inc[3] = PFS_MUL(r.vcoef, PFS_SUB(vj.x, me.pv.x));
+    inc[4] = PFS_MUL(r.vcoef, PFS_SUB(vj.y, me.pv.y));
+    inc[5] = PFS_MUL(r.vcoef, PFS_SUB(vj.z, me.pv.z));
+    inc[6] = inc[7] = inc[8] = 0.0f;
     const float nnd = rrj.y;
+    if (near_vanishes(P, me, nnd)) return;
     const float shared_near = PFS_MUL(PFS_ADD(me.near_pressure, PFS_MUL(nnd, P.kn)), 0.5f);
     const float nslope = PFS_MUL(a2, P.near_slope_scale);
     const float ncoef = PFS_DIV(PFS_MUL(PFS_MUL(shared_near, nslope), m), nnd);
-    inc[6] = PFS_MUL(ncoef, dirx);
-    inc[7] = PFS_MUL(ncoef, diry);
-    inc[8] = PFS_MUL(ncoef, dirz);
+    inc[6] = PFS_MUL(ncoef, r.x);
+    inc[7] = PFS_MUL(ncoef, r.y);
+    inc[8] = PFS_MUL(ncoef, r.z);
 }
 
 // Accumulator `lane` (0..5: fpx fpy fpz fvx fvy fvz) takes one candidate's
@@ -960,6 +963,10 @@ int nbr_variant() {
     return v;
 }
 
+bool small_world(const DevParams& P, const StepBuffers& b) {
+    return (b.fp16 || b.variant == NBR_FLAT) && !b.sr.scenes && !P.geo && P.n <= SMALL_SLOTS;
+}
+
 // Launch kernel K in its one-world or batch form.
 #define PFS_LAUNCH(K, grid, ...)                                          \
     do {                                                                  \
@@ -973,6 +980,7 @@ cudaError_t launch_density(const DevParams& P, const StepBuffers& b, cudaStream_
     if (P.n == 0) return cudaSuccess;
     const unsigned g = grid_for(P.n, NBR_THREADS);
     if (b.variant == NBR_STAGED && P.staged && !b.sr.scenes) return launch_density_staged(P, b, b.fast != 0, s);
+    if (small_world(P, b)) return launch_density_small(P, b, Dens32{b.xp}, s);
     switch (b.variant) {
         case NBR_SIMPLE:
             PFS_LAUNCH(k_density_simple, g, b.xp, b.table, b.order, b.rr, b.err);

@@ -261,6 +261,116 @@ __global__ void k_identity(const uint32_t* __restrict__ keys_in, uint32_t n,
     }
 }
 
+// A sort of at most SMALL_KEYS keys by one thread block: the keys and values stay
+// on the SM between passes.  The same ranks as k_sort_onesweep (warp match in key
+// order, per-warp digit counts), so the same stable order.  At these sizes the
+// sweeps of the general sort are latency: a memset and P + 1 launches of 4 to 9 us
+// each (24 us per sort for 2,047 keys and for 8,192; here 10 and 22, and 41 against
+// 33 for 16,384, where the general sort takes over).
+constexpr int SMALL_THREADS = 1024;
+constexpr int SMALL_WARPS = SMALL_THREADS / 32;
+constexpr uint32_t SMALL_KEYS = 8192;
+// per-warp counts, digit bases, and the keys and values
+constexpr size_t SMALL_SMEM = ((size_t)SMALL_WARPS * RADIX + RADIX + 2 * SMALL_KEYS) * 4;
+
+template <int IPT>
+__global__ void __launch_bounds__(SMALL_THREADS, 1)
+k_sort_small(const uint32_t* __restrict__ keys_in, uint32_t n, int passes, uint32_t* __restrict__ keys_out,
+             uint32_t* __restrict__ vals_out) {
+    extern __shared__ uint32_t s_mem[];
+    uint32_t* s_warp = s_mem;                          // [SMALL_WARPS][RADIX]
+    uint32_t* s_base = s_warp + SMALL_WARPS * RADIX;   // [RADIX]
+    uint32_t* s_keys = s_base + RADIX;                 // [SMALL_KEYS]
+    uint32_t* s_vals = s_keys + SMALL_KEYS;            // [SMALL_KEYS]
+    __shared__ uint32_t s_part[RADIX / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t base = (uint32_t)warp * (32 * IPT) + (uint32_t)lane;
+    const uint32_t lt = lanemask_lt();
+    uint32_t k[IPT], v[IPT], r[IPT];
+#pragma unroll
+    for (int it = 0; it < IPT; it++) {
+        const uint32_t i = base + 32u * it;
+        k[it] = i < n ? __ldg(keys_in + i) : 0u;
+        v[it] = i;
+    }
+    for (int p = 0; p < passes; p++) {
+        for (int i = threadIdx.x; i < SMALL_WARPS * RADIX; i += SMALL_THREADS) s_warp[i] = 0u;
+        __syncthreads();
+        uint32_t* mine = s_warp + warp * RADIX;
+#pragma unroll
+        for (int it = 0; it < IPT; it++) {
+            const bool valid = base + 32u * it < n;
+            const uint32_t d = valid ? (k[it] >> (8 * p)) & (RADIX - 1) : RADIX;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            const int leader = __ffs(peers) - 1;
+            uint32_t before = 0;
+            if (valid && lane == leader) {
+                before = mine[d];
+                mine[d] = before + __popc(peers);
+            }
+            before = __shfl_sync(0xffffffffu, before, leader);
+            r[it] = before + __popc(peers & lt);
+        }
+        __syncthreads();
+        // per digit: offsets of the warps (key order is warp-major) and the base
+        uint32_t cnt = 0, incl = 0;
+        if (threadIdx.x < RADIX) {
+#pragma unroll 8
+            for (int w = 0; w < SMALL_WARPS; w++) {
+                const uint32_t c = s_warp[w * RADIX + threadIdx.x];
+                s_warp[w * RADIX + threadIdx.x] = cnt;
+                cnt += c;
+            }
+            incl = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (lane == 31) s_part[warp] = incl;
+        }
+        __syncthreads();
+        if (threadIdx.x < RADIX) {
+            uint32_t before = 0;
+            for (int w = 0; w < warp; w++) before += s_part[w];
+            s_base[threadIdx.x] = before + incl - cnt;
+        }
+        __syncthreads();
+        const bool last = p == passes - 1;
+#pragma unroll
+        for (int it = 0; it < IPT; it++) {
+            if (base + 32u * it >= n) continue;
+            const uint32_t d = (k[it] >> (8 * p)) & (RADIX - 1);
+            const uint32_t pos = s_base[d] + mine[d] + r[it];  // < n: ranks of n keys
+            s_keys[pos] = k[it];
+            s_vals[pos] = v[it];
+        }
+        __syncthreads();
+        if (last) break;
+#pragma unroll
+        for (int it = 0; it < IPT; it++) {
+            const uint32_t i = base + 32u * it;
+            if (i < n) {
+                k[it] = s_keys[i];
+                v[it] = s_vals[i];
+            }
+        }
+    }
+    for (uint32_t i = threadIdx.x; i < n; i += SMALL_THREADS) {
+        keys_out[i] = s_keys[i];
+        vals_out[i] = s_vals[i];
+    }
+}
+
+cudaError_t sort_small(const uint32_t* keys_in, uint32_t n, int passes, uint32_t* keys_out, uint32_t* vals_out,
+                       cudaStream_t stream) {
+    auto k = n <= 2048u ? k_sort_small<2> : (n <= 4096u ? k_sort_small<4> : k_sort_small<8>);
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SMEM);
+    if (e != cudaSuccess) return e;
+    k<<<1, SMALL_THREADS, SMALL_SMEM, stream>>>(keys_in, n, passes, keys_out, vals_out);
+    return cudaGetLastError();
+}
+
 // Upsweep grid: a few blocks per SM, striding over the keys (measured: one
 // block per SM leaves the pass latency-bound, 21 us against 14 us at 1M).
 unsigned upsweep_blocks(uint32_t n) {
@@ -291,7 +401,7 @@ size_t sort_scratch_words(uint32_t n, int key_bits) {
 
 int sort_launches(uint32_t n) {
     const int p = sort_passes(n);
-    return p == 0 ? 1 : 1 + p;
+    return p == 0 || n <= SMALL_KEYS ? 1 : 1 + p;
 }
 
 cudaError_t sort_pairs(const uint32_t* keys_in, uint32_t n, int key_bits, uint32_t* keys_out,
@@ -304,6 +414,7 @@ cudaError_t sort_pairs(const uint32_t* keys_in, uint32_t n, int key_bits, uint32
         return cudaGetLastError();
     }
     if (passes > MAX_PASSES) return cudaErrorInvalidValue;
+    if (n <= SMALL_KEYS) return sort_small(keys_in, n, passes, keys_out, vals_out, stream);
     const uint32_t tiles = sort_tiles(n);
     uint32_t* ghist = scratch;
     uint32_t* tile_ctr = scratch + (size_t)MAX_PASSES * RADIX;

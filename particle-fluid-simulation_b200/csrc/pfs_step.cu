@@ -75,7 +75,7 @@ k_reorder(DevParams P0, SceneRef sr, const uint32_t* __restrict__ skeys, const u
     const uint32_t k = skeys[s];
     if (p >= n || k >= n) {
         atomicOr(err, p >= n ? ERR_PERM_RANGE : ERR_KEY_RANGE);
-        bucket[s] = 0xffffffffu;
+        if (bcount) bucket[s] = 0xffffffffu;
         return;
     }
     const float4 xo = x[p];
@@ -90,9 +90,11 @@ k_reorder(DevParams P0, SceneRef sr, const uint32_t* __restrict__ skeys, const u
     if (rec) rec[s] = make_record(P, pos, vo);  // FP16-cell form
     // block of x* for the neighbour passes' processing order (any order gives
     // the same results; this one keeps a warp's neighbours in cache)
-    const uint32_t blk = spatial_bucket(P, pos.x, pos.y, pos.z);
-    bucket[s] = blk;
-    brank[s] = atomicAdd(bcount + blk, 1u);
+    if (bcount) {
+        const uint32_t blk = spatial_bucket(P, pos.x, pos.y, pos.z);
+        bucket[s] = blk;
+        brank[s] = atomicAdd(bcount + blk, 1u);
+    }
     if (ids) ids_s[s] = ids[p];
     const bool head = (s == 0) || (skeys[s - 1] != k);
     const bool tail = (s == n - 1) || (skeys[s + 1] != k);
@@ -250,16 +252,20 @@ cudaError_t launch_sort(const DevParams& P, const StepBuffers& b, cudaStream_t s
 cudaError_t launch_reorder(const DevParams& P, const StepBuffers& b, cudaStream_t s) {
     if (P.n == 0) return cudaSuccess;
     const unsigned g = grid_for(P.n, ELEM_THREADS);
+    // a small world's neighbour passes take the slots as they are
+    const bool ordered = !small_world(P, b);
+    uint32_t* bcount = ordered ? b.bcount : nullptr;
     if (b.sr.scenes)
         k_reorder<true><<<g, ELEM_THREADS, 0, s>>>(P, b.sr, b.skeys, b.perm, b.x, b.v, b.ids, b.xs,
                                                    b.vs, b.xp, b.vp, b.ids_s, b.table, b.bucket,
-                                                   b.brank, b.bcount, b.bcounter, b.scanq_n, b.rec,
+                                                   b.brank, bcount, b.bcounter, b.scanq_n, b.rec,
                                                    b.st_counters, b.err);
     else
         k_reorder<false><<<g, ELEM_THREADS, 0, s>>>(P, b.sr, b.skeys, b.perm, b.x, b.v, b.ids, b.xs,
                                                     b.vs, b.xp, b.vp, b.ids_s, b.table, b.bucket,
-                                                    b.brank, b.bcount, b.bcounter, b.scanq_n, b.rec,
+                                                    b.brank, bcount, b.bcounter, b.scanq_n, b.rec,
                                                     b.st_counters, b.err);
+    if (!ordered) return cudaGetLastError();
     const uint32_t nb = b.nblocks;
     if (P.staged) {
         // fine buckets: each staged block's cells get one contiguous segment
@@ -291,10 +297,10 @@ cudaError_t launch_integrate(const DevParams& P, const StepBuffers& b, cudaStrea
     return cudaGetLastError();
 }
 
-// sort + reorder/bucket (3) + density + force + integrate (+ the two
-// grid-search passes)
-int substep_launches(uint32_t n, bool geo) {
-    return n == 0 ? 0 : sort_launches(n) + 6 + (geo ? 2 : 0);
+// sort + reorder/bucket (3; a small world 1) + density + force + integrate (+ the
+// two grid-search passes)
+int substep_launches(uint32_t n, bool geo, bool small) {
+    return n == 0 ? 0 : sort_launches(n) + (small ? 4 : 6) + (geo ? 2 : 0);
 }
 
 }  // namespace pfs

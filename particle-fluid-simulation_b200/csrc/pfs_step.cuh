@@ -58,6 +58,7 @@ struct StepBuffers {
     // the spatial-order blocks of all scenes together
     SceneRef sr;
     uint32_t nblocks;
+    uint32_t fp16;      // the FP16-cell form
     // FP16-cell form: 16-byte neighbour records the reorder writes (null for
     // the FP32 form)
     uint4* rec;
@@ -181,6 +182,12 @@ enum { NBR_SIMPLE = 0, NBR_COMPACT = 1, NBR_LIST = 2, NBR_FLAT = 3, NBR_STAGED =
 int nbr_variant();
 
 // Launches one substep issues (sort included; geo: grid search in use).
-int substep_launches(uint32_t n, bool geo);
+int substep_launches(uint32_t n, bool geo, bool small);
+// The step's density pass runs one warp per slot (pfs_small.cuh), without the
+// spatial order.  SMALL_SLOTS: where the flat walk and its order become faster
+// (step of the dam break, three substeps: 16,384 particles 0.25 to 0.20 ms, 32,768
+// 0.30 ms both ways).
+constexpr uint32_t SMALL_SLOTS = 24576;
+bool small_world(const DevParams& P, const StepBuffers& b);
 
 }  // namespace pfs

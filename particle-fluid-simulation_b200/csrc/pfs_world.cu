@@ -440,6 +440,7 @@ int carve(pfs_world* w) {
     set_cells(w);
     b.fast = w->params.precision == PFS_FP32_FAST ? 1 : 0;
     b.sr = SceneRef{nullptr, nullptr};
+    b.fp16 = w->params.precision == PFS_FP16_CELL ? 1u : 0u;
     b.nblocks = spatial_blocks(w->dp);
     // the FP16-cell form has one shape, the list shape's
     b.variant = w->params.precision == PFS_FP16_CELL ? (int)NBR_LIST : nbr_variant();
@@ -1248,7 +1249,7 @@ int pfs_world_stage_times(pfs_world* w, pfs_stage_times* out) {
 }
 
 int pfs_world_launches_per_substep(const pfs_world* w) {
-    return w ? substep_launches(w->n, w->dp.geo != 0) : 0;
+    return w ? substep_launches(w->n, w->dp.geo != 0, small_world(w->dp, w->b)) : 0;
 }
 
 int pfs_world_debug_substep(pfs_world* w, pfs_debug_substep* o) {
