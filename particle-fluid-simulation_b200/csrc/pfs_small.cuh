@@ -8,9 +8,7 @@
 // 0 .. 26 look a slot's ranges up together, the lanes hold 32 candidates at a time
 // and evaluate the in-range terms together, and only the sums run in order: 10 us
 // for 2,047 slots, 16 for 16,384, and the slots are their own processing order.
-// (24 us against the flat walk's 35 at 32,768, where the force pass's gathers in
-// key order take the difference back.)  Candidates, terms, order, lists and queue
-// are the flat walk's.
+// Candidates, terms, order, lists and queue are the flat walk's.
 #pragma once
 
 #include <cstdint>

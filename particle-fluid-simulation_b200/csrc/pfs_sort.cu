@@ -40,8 +40,14 @@ namespace {
 
 constexpr int SORT_THREADS = 256;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
-constexpr int SORT_IPT = 16;
-constexpr int SORT_TILE = SORT_THREADS * SORT_IPT;
+// Keys per thread of a tile: 16, fewer where 4096-key tiles would leave SMs idle
+// (a tile's ranks are serial, one warp match per key of a thread, so a small sort
+// takes as long as its tiles do): 16,384 keys 33 us with 16 per thread, 24 with 4;
+// 300,000 keys 51 us with 16, 44 with 8; 1M keys 70 us with 16, 77 with 8.
+constexpr uint32_t SORT_MAX_4 = 1u << 17;
+constexpr uint32_t SORT_MAX_8 = 1u << 19;
+__host__ __device__ constexpr int sort_ipt(uint32_t n) { return n <= SORT_MAX_4 ? 4 : (n <= SORT_MAX_8 ? 8 : 16); }
+__host__ __device__ constexpr uint32_t sort_tile(uint32_t n) { return (uint32_t)SORT_THREADS * sort_ipt(n); }
 constexpr int RADIX = 256;
 constexpr int MAX_PASSES = 4;
 constexpr uint32_t LB_AGG = 1u << 30;
@@ -120,12 +126,13 @@ k_sort_upsweep(const uint32_t* __restrict__ keys, uint32_t n, int passes,
     }
 }
 
-template <bool FIRST>
+template <bool FIRST, int SORT_IPT>
 __global__ void __launch_bounds__(SORT_THREADS, 2)
 k_sort_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                 uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n,
                 int shift, const uint32_t* __restrict__ ghist, uint32_t* __restrict__ tile_ctr,
                 uint32_t* __restrict__ look, uint32_t* __restrict__ err) {
+    constexpr int SORT_TILE = SORT_THREADS * SORT_IPT;
     __shared__ uint32_t s_keys[SORT_TILE];
     __shared__ uint32_t s_vals[SORT_TILE];
     __shared__ uint32_t s_warp[SORT_WARPS][RADIX];
@@ -381,7 +388,7 @@ unsigned upsweep_blocks(uint32_t n) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (sms <= 0) sms = 148;
     }
-    const unsigned want = (n + SORT_TILE - 1) / SORT_TILE;
+    const unsigned want = sort_tiles(n);
     return std::max(1u, std::min(want, (unsigned)(4 * sms)));
 }
 
@@ -391,11 +398,13 @@ int sort_key_bits(uint32_t n) { return n <= 1 ? 0 : 32 - __builtin_clz(n - 1u); 
 
 int sort_passes(uint32_t n) { return (sort_key_bits(n) + 7) / 8; }
 
-uint32_t sort_tiles(uint32_t n) { return (n + SORT_TILE - 1) / SORT_TILE; }
+uint32_t sort_tiles(uint32_t n) { return (n + sort_tile(n) - 1) / sort_tile(n); }
 
 size_t sort_scratch_words(uint32_t n, int key_bits) {
     const int passes = (key_bits + 7) / 8;
-    const size_t tiles = sort_tiles(n) > 0 ? sort_tiles(n) : 1;
+    // (smaller sorts, in the same scratch, have smaller tiles)
+    const size_t tiles = std::max({1u, sort_tiles(n), sort_tiles(std::min(n, SORT_MAX_4)),
+                                   sort_tiles(std::min(n, SORT_MAX_8))});
     return HEADER_WORDS + (size_t)(passes > 0 ? passes : 1) * tiles * RADIX;
 }
 
@@ -433,12 +442,11 @@ cudaError_t sort_pairs(const uint32_t* keys_in, uint32_t n, int key_bits, uint32
         uint32_t* vout = to_final ? vals_out : vals_tmp;
         const int shift = 8 * p;
         uint32_t* lp = look + (size_t)p * tiles * RADIX;
-        if (p == 0)
-            k_sort_onesweep<true><<<tiles, SORT_THREADS, 0, stream>>>(
-                kin, vin, kout, vout, n, shift, ghist + p * RADIX, tile_ctr + p, lp, err);
-        else
-            k_sort_onesweep<false><<<tiles, SORT_THREADS, 0, stream>>>(
-                kin, vin, kout, vout, n, shift, ghist + p * RADIX, tile_ctr + p, lp, err);
+        const int ipt = sort_ipt(n);
+        auto k = p == 0 ? (ipt == 4 ? k_sort_onesweep<true, 4> : (ipt == 8 ? k_sort_onesweep<true, 8> : k_sort_onesweep<true, 16>))
+                        : (ipt == 4 ? k_sort_onesweep<false, 4>
+                                    : (ipt == 8 ? k_sort_onesweep<false, 8> : k_sort_onesweep<false, 16>));
+        k<<<tiles, SORT_THREADS, 0, stream>>>(kin, vin, kout, vout, n, shift, ghist + p * RADIX, tile_ctr + p, lp, err);
         kin = kout;
         vin = vout;
     }

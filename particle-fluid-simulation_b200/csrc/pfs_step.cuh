@@ -185,9 +185,9 @@ int nbr_variant();
 int substep_launches(uint32_t n, bool geo, bool small);
 // The step's density pass runs one warp per slot (pfs_small.cuh), without the
 // spatial order.  SMALL_SLOTS: where the flat walk and its order become faster
-// (step of the dam break, three substeps: 16,384 particles 0.25 to 0.20 ms, 32,768
-// 0.30 ms both ways).
-constexpr uint32_t SMALL_SLOTS = 24576;
+// (reorder, density and force of one substep, dam break and slab: 16,384 slots 40
+// against 60 us, 32,768 51 against 65, 131,072 160 against 127).
+constexpr uint32_t SMALL_SLOTS = 49152;
 bool small_world(const DevParams& P, const StepBuffers& b);
 
 }  // namespace pfs

@@ -12,7 +12,7 @@ from test_gpu_parity import _assert_bits_equal, _check_substep, _uniform_scene
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [1, 31, 2047, 2048, 2049, 4096, 4097, 8192, 8193, 24576, 24577])
+@pytest.mark.parametrize("n", [1, 31, 2047, 2048, 2049, 4096, 4097, 8192, 8193, 49152, 49153])
 def test_small_world_substep(cuda_device, monkeypatch, n):
     monkeypatch.setenv("PFS_NEIGHBOR_SEARCH", "table")
     pfs, ora = load_package(), load_oracle()
@@ -26,7 +26,7 @@ def test_small_world_substep(cuda_device, monkeypatch, n):
     _check_substep(pfs, ora, p, pos, vel)
 
 
-@pytest.mark.parametrize("n", [1, 500, 4097, 24576])
+@pytest.mark.parametrize("n", [1, 500, 4097, 49152])
 def test_small_world_fp16_equals_list_walk(cuda_device, n):
     """The FP16-cell form's small-world sums equal its grid search's."""
     pfs = load_package()
