@@ -38,6 +38,19 @@ namespace {
 constexpr int FLAT_THREADS = 128;       // threads per block (column in 7 bits)
 constexpr int FLAT_RCAP = 28;           // range words per particle (a multiple of 4)
 constexpr uint32_t FLAT_LEN_MAX = 127;  // candidates per range word
+// Deferred terms per lane, thread blocks on an SM, and the share of the SM's
+// memory (percent) kept as shared memory.  What bounds the walk is the L1: a
+// warp's candidates are read again by the block's other warps and by its
+// neighbours, and every miss waits in the load queue ahead of the walk's
+// shared-memory words.  As many blocks as fit the largest share (10 of 22 KB)
+// leave the L1 28 KB, where 25% of its sectors hit; 8 blocks of 20 KB leave it
+// 92 KB.  Density pass of 4,194,304 particles in colliding blocks 1,960 -> 970
+// us (FP16 cells 1,085 -> 1,044), of the 1,000,000-particle slab 357 -> 352
+// (402 -> 400).  Shares of 80% (60 KB of L1): 1,031 and 340 us; 56%: 1,104 and
+// 389 us.
+constexpr int FLAT_CAP = 8;
+constexpr int FLAT_BLOCKS = 8;
+constexpr int FLAT_CARVEOUT = 64;
 static_assert(PFS_MAX_PARTICLES <= (1u << 24), "packed range start");
 static_assert(FLAT_RCAP % 4 == 0, "moved in four parts");
 
@@ -255,6 +268,11 @@ __device__ __forceinline__ void flat_walk(const FlatShared& S, int32_t tot, int3
         walk(std::true_type{});
     else
         walk(std::false_type{});
+}
+
+template <class K>
+cudaError_t flat_carveout(K kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, FLAT_CARVEOUT);
 }
 
 // The scan queue: positions whose density pass wrote no usable list.

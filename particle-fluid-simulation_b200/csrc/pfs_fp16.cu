@@ -82,8 +82,6 @@ __device__ __forceinline__ float2 density16_finish(const DevParams& P, float s2,
 // their order are those of the 27-cell table walk (density16_scan_one), so
 // the compensated sums, in that order, and the list and queue decisions are
 // the same bits as a particle's own walk.
-constexpr int D16_CAP = 12;  // deferred q2 per lane
-
 // Density sums of one particle by its own 27-cell walk from global memory
 // in the reference's order: the fallback of the flat shape.
 __device__ __forceinline__ void density16_scan_one(const DevParams& P, const float4 sp, const Unpacked& me,
@@ -132,7 +130,7 @@ __device__ __forceinline__ void density16_scan_one(const DevParams& P, const flo
 }
 
 template <bool BATCH>
-__global__ void __launch_bounds__(NBR_THREADS, BATCH ? 8 : 9)
+__global__ void __launch_bounds__(NBR_THREADS, FLAT_BLOCKS)
 k_density16_flat(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const uint4* __restrict__ rec,
                  const int2* __restrict__ table, const uint32_t* __restrict__ order,
                  float2* __restrict__ rr, int32_t* __restrict__ nlist, int32_t* __restrict__ ncount,
@@ -140,7 +138,7 @@ k_density16_flat(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const
                  uint32_t* __restrict__ err) {
     static_assert(NBR_THREADS == FLAT_THREADS, "the flat walk's block");
     __shared__ FlatShared S;
-    __shared__ float s_q2[D16_CAP][NBR_THREADS];  // per thread: deferred q2
+    __shared__ float s_q2[FLAT_CAP][NBR_THREADS];  // per thread: deferred q2
     const int tid = threadIdx.x;
     const uint32_t n = P0.n;
     uint32_t key = flat_ranges<BATCH>(P0, sr, xp, table, order, err, S);
@@ -157,7 +155,7 @@ k_density16_flat(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const
     const int32_t self = (int32_t)i;
     float s2 = 0.0f, c2 = 0.0f, s3 = 0.0f, c3 = 0.0f;
     float* dp = &s_q2[0][tid];
-    float* const dfull = &s_q2[D16_CAP - 1][tid];
+    float* const dfull = &s_q2[FLAT_CAP - 1][tid];
     int32_t cnt = 0;
     const int32_t lcap1 = (int32_t)P.list_cap - 1;
     auto test = [&](const uint4 q, int32_t jq, bool fq, bool valid) {
@@ -181,7 +179,7 @@ k_density16_flat(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const
     // all lanes drain together once one of them has no room for a pair
     auto drain_if_full = [&]() {
         if (__any_sync(0xffffffffu, dp >= dfull)) {
-            for (int c = 0; c < D16_CAP; c++)
+            for (int c = 0; c < FLAT_CAP; c++)
                 if (&s_q2[c][tid] < dp) term(s_q2[c][tid]);
             dp = &s_q2[0][tid];
         }
@@ -787,6 +785,8 @@ cudaError_t launch_density_fp16(const DevParams& P, const StepBuffers& b, const 
     const unsigned g = grid_for(P.n, NBR_THREADS);
     if (!b.all_geo) {
         auto k = b.sr.scenes ? k_density16_flat<true> : k_density16_flat<false>;
+        const cudaError_t e = flat_carveout(k);
+        if (e != cudaSuccess) return e;
         k<<<g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, f.rec, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
                                     b.scanq_n, b.err);
     }

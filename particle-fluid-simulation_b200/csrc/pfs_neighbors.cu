@@ -442,10 +442,8 @@ k_density_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const i
 // written as they are found.  Appends store unconditionally and advance the
 // count by the predicate.  A particle whose ranges do not fit the walk's
 // stage walks the table from global memory (density_scan_one).
-constexpr int FLAT_CAP = 14;  // buffered density terms per lane
-
 template <bool BATCH>
-__global__ void __launch_bounds__(NBR_THREADS, BATCH ? 8 : 10)
+__global__ void __launch_bounds__(NBR_THREADS, FLAT_BLOCKS)
 k_density_flat(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const int2* __restrict__ table,
                const uint32_t* __restrict__ order, float2* __restrict__ rr,
                int32_t* __restrict__ nlist, int32_t* __restrict__ ncount,
@@ -990,12 +988,16 @@ cudaError_t launch_density(const DevParams& P, const StepBuffers& b, cudaStream_
             break;
         default:
             if (!b.all_geo) {
-                if (b.variant == NBR_FLAT)
-                    PFS_LAUNCH(k_density_flat, g, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
-                               b.scanq_n, b.err);
-                else
+                if (b.variant == NBR_FLAT) {
+                    auto k = b.sr.scenes ? k_density_flat<true> : k_density_flat<false>;
+                    const cudaError_t e = flat_carveout(k);
+                    if (e != cudaSuccess) return e;
+                    k<<<g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
+                                                b.scanq_n, b.err);
+                } else {
                     PFS_LAUNCH(k_density_list, g, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
                                b.scanq_n, b.err);
+                }
             }
             if (b.geo_any) {
                 const cudaError_t e = launch_cells(P, b, Dens32{b.xp}, s);
