@@ -114,7 +114,7 @@ void drop_graph(pfs_batch* B) {
 }
 
 size_t batch_arena_bytes(uint32_t cap_n, uint32_t cap_s, int precision, uint32_t blocks_cap) {
-    size_t b = world_arena_bytes(cap_n, 0, precision, blocks_cap, NLIST_CAP_MAX, 0);
+    size_t b = world_arena_bytes(cap_n, 0, precision, blocks_cap, NLIST_CAP_MAX, 0, precision != PFS_FP16_CELL);
     b += (size_t)cap_s * sizeof(DevParams) + (size_t)cap_n * 4 /*sid*/ + ((size_t)cap_s + 1) * 4;
     b += 2 * (size_t)cap_n * 16; /* x0 v0 */
     b += ((size_t)blocks_cap / 256 + 1) * 4; /* cvshift */
@@ -268,6 +268,7 @@ int pfs_batch_create(uint32_t max_particles, uint32_t max_scenes, int32_t precis
     b.xp = (float4*)a.take(f4);
     b.vp = (float4*)a.take(f4);
     b.rr = (float2*)a.take((size_t)max_particles * 8);
+    b.fr = precision == PFS_FP16_CELL ? nullptr : (float4*)a.take(2 * f4);
     b.keys = (uint32_t*)a.take(u);
     b.skeys = (uint32_t*)a.take(u);
     b.perm = (uint32_t*)a.take(u);
@@ -297,7 +298,7 @@ int pfs_batch_create(uint32_t max_particles, uint32_t max_scenes, int32_t precis
     b.nblocks = 0;
     b.fp16 = B->precision == PFS_FP16_CELL ? 1u : 0u;
     b.variant = B->precision == PFS_FP16_CELL ? (int)NBR_LIST : nbr_variant();
-    bool ok = b.x && b.v && b.xs && b.vs && b.xp && b.vp && b.rr && b.keys && b.skeys && b.perm &&
+    bool ok = (b.fr || precision == PFS_FP16_CELL) && b.x && b.v && b.xs && b.vs && b.xp && b.vp && b.rr && b.keys && b.skeys && b.perm &&
               b.keys_tmp && b.vals_tmp && b.sort_scratch && b.table && b.err && b.order &&
               b.bucket && b.brank && b.bcount && b.boffset && b.bcounter && b.nlist && b.ncount &&
               b.scanq && b.scanq_n && b.clist && b.cvshift && B->d_scenes && B->d_sid && B->d_offs && B->x0 && B->v0;

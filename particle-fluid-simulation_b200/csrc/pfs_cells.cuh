@@ -303,7 +303,7 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
                 const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ order,
                 const uint32_t* __restrict__ clist, const uint32_t* __restrict__ cvshift,
                 const uint32_t* __restrict__ bcount, const uint32_t* __restrict__ boffset, CellsLayout lay,
-                float2* __restrict__ rr, int32_t* __restrict__ nlist,
+                float2* __restrict__ rr, float4* __restrict__ fr, int32_t* __restrict__ nlist,
                 int32_t* __restrict__ ncount, uint32_t* __restrict__ scanq, uint32_t* __restrict__ scanq_n,
                 uint32_t* __restrict__ slowq, uint32_t* __restrict__ err) {
     extern __shared__ float4 s_dyn[];
@@ -606,7 +606,7 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
                 }
                 const bool scan = done && lcnt > lcap;
                 if (done) {
-                    rr[self] = sum.finish(P);
+                    put_rr(rr, fr, self, sum.finish(P));
                     ncount[tm] = scan ? -1 : (int32_t)lcnt;
                 }
                 if (scan) {  // the force pass scans for itself
@@ -643,7 +643,7 @@ cudaError_t launch_cells(const DevParams& P, const StepBuffers& b, const F& form
     if (e != cudaSuccess) return e;
     const unsigned grid = std::max(1u, std::min(cells_grid(k, dyn), P.n));
     k<<<grid, CELLS_THREADS, dyn, s>>>(P, b.sr, form, b.xp, b.skeys, b.order, b.clist, b.cvshift, b.bcount, b.boffset,
-                                       lay, b.rr, b.nlist, b.ncount, b.scanq, b.scanq_n, b.keys_tmp, b.err);
+                                       lay, b.rr, b.records(), b.nlist, b.ncount, b.scanq, b.scanq_n, b.keys_tmp, b.err);
     return cudaGetLastError();
 }
 

@@ -266,4 +266,11 @@ uint32_t spatial_blocks(const DevParams& P);
 // Coarsen the spatial order until at most `cap` buckets remain.
 void fit_spatial_blocks(DevParams* P, uint32_t cap);
 
+// A particle's densities: the array the host reads, and the last two floats of
+// its neighbour record where there is one (StepBuffers::fr).
+__device__ __forceinline__ void put_rr(float2* __restrict__ rr, float4* __restrict__ fr, uint32_t i, float2 d) {
+    rr[i] = d;
+    if (fr) *(reinterpret_cast<float2*>(fr) + 4 * (size_t)i + 3) = d;
+}
+
 }  // namespace pfs

@@ -341,7 +341,6 @@ k_map_cells(DevParams P, MapArgs A, CellsLayout lay, const float4* __restrict__ 
     uint32_t* zone = reinterpret_cast<uint32_t*>(s_dyn + lay.entries) + warp * (cells_warp_bytes(lay) / 4);
     uint2* ballots = reinterpret_cast<uint2*>(zone);                      // [words]
     uint16_t* at = reinterpret_cast<uint16_t*>(zone + 2u * lay.words);     // [slots][64]
-    const float h = P.h;
     const uint32_t nblk = *listed;
     const int3 dim0 = make_int3(1 << P.bsx, 1 << P.bsy, 1 << P.bsz);
     const int cells = dim0.x * dim0.y * dim0.z;

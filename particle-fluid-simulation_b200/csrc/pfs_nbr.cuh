@@ -146,6 +146,21 @@ struct ForceAcc {
     float fpx, fpy, fpz, fvx, fvy, fvz;
 };
 
+// A neighbour of the force pass: x*, (density, near density), v.
+struct ForceNbr {
+    float4 x, v;
+    float2 r;
+};
+
+// One 32-byte load (x* y* z* v.x | v.y v.z density near).
+__device__ __forceinline__ ForceNbr force_nbr(const float4* __restrict__ fr, int32_t j) {
+    float a[8];
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]), "=f"(a[7])
+        : "l"(fr + 2 * (size_t)j));
+    return ForceNbr{make_float4(a[0], a[1], a[2], 1.0f), make_float4(a[3], a[4], a[5], 0.0f), make_float2(a[6], a[7])};
+}
+
 struct ForceSelf {
     float4 sp, pv;
     float my_pressure_term, near_pressure;

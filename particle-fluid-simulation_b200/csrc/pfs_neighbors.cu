@@ -249,12 +249,15 @@ k_force_slab(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const flo
 // through the queue of positions without a list (full scans, long latency
 // chains, issued first so they overlap the list work); the others evaluate
 // one listed particle per thread, a block's 128 positions in ascending list
-// length.
-template <bool BATCH, bool FAST>
-__global__ void __launch_bounds__(NBR_THREADS)
+// length.  PACKED: a neighbour is one 32-byte record (StepBuffers::records has
+// the rule).  Latency binds it: six blocks on an SM (80 registers) and four
+// neighbours in flight; five or seven blocks: 300,000 dense particles 906 and 907
+// us against 815, 1,000,000-particle slab 169 and 156 against 149.
+template <bool BATCH, bool FAST, bool PACKED>
+__global__ void __launch_bounds__(NBR_THREADS, 6)
 k_force_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const float4* __restrict__ vp,
              const float4* __restrict__ vs, const float2* __restrict__ rr,
-             const int2* __restrict__ table, const uint32_t* __restrict__ order,
+             const float4* __restrict__ fr, const int2* __restrict__ table, const uint32_t* __restrict__ order,
              const int32_t* __restrict__ nlist, const int32_t* __restrict__ ncount,
              const uint32_t* __restrict__ scanq, const uint32_t* __restrict__ scanq_n,
              uint32_t qblocks, uint32_t in_order, float4* __restrict__ vout,
@@ -300,25 +303,22 @@ k_force_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const flo
     for (int32_t k = 0; k < cnt; k += 4) {
         int32_t j[4] = {jn[0], jn[1], jn[2], jn[3]};
         indices(k + 4);
-        float4 q[4], vj[4];
-        float2 rj[4];
+        ForceNbr q[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             if ((uint32_t)j[u] >= n) {
                 atomicOr(err, ERR_TABLE_RANGE);
                 j[u] = (int32_t)i;
             }
-            q[u] = __ldg(xp + j[u]);
-            vj[u] = __ldg(vs + j[u]);
-            rj[u] = __ldg(rr + j[u]);
+            q[u] = PACKED ? force_nbr(fr, j[u]) : ForceNbr{__ldg(xp + j[u]), __ldg(vs + j[u]), __ldg(rr + j[u])};
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             if constexpr (FAST)
-                force_term_fast(P, me, make_float4(q[u].x, q[u].y, q[u].z, rj[u].x),
-                                make_float4(vj[u].x, vj[u].y, vj[u].z, rj[u].y), f);
+                force_term_fast(P, me, make_float4(q[u].x.x, q[u].x.y, q[u].x.z, q[u].r.x),
+                                make_float4(q[u].v.x, q[u].v.y, q[u].v.z, q[u].r.y), f);
             else
-                force_term_pre(P, me, q[u], rj[u], vj[u], f);
+                force_term_pre(P, me, q[u].x, q[u].r, q[u].v, f);
         }
     }
     __stcs(vout + i, force_finish(P, f, __ldcs(vs + i), rri.x));
@@ -335,7 +335,7 @@ constexpr int DENS_CAP = 32;
 template <bool BATCH>
 __global__ void __launch_bounds__(NBR_THREADS, 8)
 k_density_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const int2* __restrict__ table,
-                const uint32_t* __restrict__ order, float2* __restrict__ rr,
+                const uint32_t* __restrict__ order, float2* __restrict__ rr, float4* __restrict__ fr,
                 int32_t* __restrict__ nlist, int32_t* __restrict__ ncount,
                 uint32_t* __restrict__ scanq, uint32_t* __restrict__ scanq_n,
                 uint32_t* __restrict__ err) {
@@ -419,7 +419,7 @@ k_density_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const i
     for (int k = 0; k < cd; k++) density_term(s_dd[k][threadIdx.x], h, m, total, total_near);
     const bool scan = !(list_ok && cnt <= (int32_t)P.list_cap);
     ncount[t] = scan ? -1 : cnt;
-    rr[i] = density_finish(P, total, total_near);
+    put_rr(rr, fr, i, density_finish(P, total, total_near));
     const uint32_t active = __activemask();
     const uint32_t want = __ballot_sync(active, scan);
     if (want) {
@@ -445,7 +445,7 @@ k_density_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const i
 template <bool BATCH>
 __global__ void __launch_bounds__(NBR_THREADS, FLAT_BLOCKS)
 k_density_flat(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const int2* __restrict__ table,
-               const uint32_t* __restrict__ order, float2* __restrict__ rr,
+               const uint32_t* __restrict__ order, float2* __restrict__ rr, float4* __restrict__ fr,
                int32_t* __restrict__ nlist, int32_t* __restrict__ ncount,
                uint32_t* __restrict__ scanq, uint32_t* __restrict__ scanq_n,
                uint32_t* __restrict__ err) {
@@ -501,7 +501,7 @@ k_density_flat(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const i
     const bool scan = live && (over || !((meta & FLAT_LIST_OK) != 0 && cnt <= (int32_t)P.list_cap));
     if (live) {
         ncount[t] = scan ? -1 : cnt;
-        rr[i] = over ? density_scan_one(P, sp, xp, table, err) : density_finish(P, total, total_near);
+        put_rr(rr, fr, i, over ? density_scan_one(P, sp, xp, table, err) : density_finish(P, total, total_near));
     }
     flat_enqueue(scan, t, scanq, scanq_n);
 }
@@ -622,7 +622,8 @@ __global__ void __launch_bounds__(GEO_WARPS * 32, 6)
 k_density_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const int2* __restrict__ table,
               const uint32_t* __restrict__ order, const uint32_t* __restrict__ bcount,
               const uint32_t* __restrict__ boffset, const uint32_t* __restrict__ slowq,
-              float2* __restrict__ rr, int32_t* __restrict__ nlist, int32_t* __restrict__ ncount, uint32_t* __restrict__ scanq,
+              float2* __restrict__ rr, float4* __restrict__ fr, int32_t* __restrict__ nlist,
+              int32_t* __restrict__ ncount, uint32_t* __restrict__ scanq,
               uint32_t* __restrict__ scanq_n, uint32_t* __restrict__ err) {
     __shared__ int32_t s_j[GEO_WARPS][GEO_DCAP];
     __shared__ float s_a[GEO_WARPS][GEO_DCAP];
@@ -790,7 +791,7 @@ k_density_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const in
         total = __shfl_sync(full, total, 0);
         total_near = __shfl_sync(full, total_near, 1);
         if (lane == 0) {
-            rr[i] = density_finish(P, total, total_near);
+            put_rr(rr, fr, i, density_finish(P, total, total_near));
             const bool scan = !(list_ok && cnt <= (int32_t)P.list_cap);
             ncount[t] = scan ? -1 : cnt;
             if (scan) {
@@ -808,7 +809,7 @@ k_density_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const in
 template <bool BATCH>
 __global__ void __launch_bounds__(GEO_WARPS * 32)
 k_force_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const float4* __restrict__ vp,
-            const float4* __restrict__ vs, const float2* __restrict__ rr,
+            const float4* __restrict__ vs, const float2* __restrict__ rr, const float4* __restrict__ fr,
             const int2* __restrict__ table, const uint32_t* __restrict__ order,
             const uint32_t* __restrict__ bcount, const uint32_t* __restrict__ boffset,
             const uint32_t* __restrict__ scanq, uint32_t* __restrict__ scanq_n,
@@ -863,7 +864,8 @@ k_force_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const floa
                 for (int k = k0 + lane; k < k1; k += 32) {
                     const int32_t j = sj[k];
                     float v[FORCE_INCS];
-                    force_incr(P, me, __ldg(xp + j), __ldg(rr + j), __ldg(vs + j), v);
+                    const ForceNbr q = fr ? force_nbr(fr, j) : ForceNbr{__ldg(xp + j), __ldg(vs + j), __ldg(rr + j)};
+                    force_incr(P, me, q.x, q.r, q.v, v);
 #pragma unroll
                     for (int c = 0; c < FORCE_INCS; c++) inc[c][k - k0] = v[c];
                 }
@@ -992,10 +994,10 @@ cudaError_t launch_density(const DevParams& P, const StepBuffers& b, cudaStream_
                     auto k = b.sr.scenes ? k_density_flat<true> : k_density_flat<false>;
                     const cudaError_t e = flat_carveout(k);
                     if (e != cudaSuccess) return e;
-                    k<<<g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
+                    k<<<g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.table, b.order, b.rr, b.records(), b.nlist, b.ncount, b.scanq,
                                                 b.scanq_n, b.err);
                 } else {
-                    PFS_LAUNCH(k_density_list, g, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
+                    PFS_LAUNCH(k_density_list, g, b.xp, b.table, b.order, b.rr, b.records(), b.nlist, b.ncount, b.scanq,
                                b.scanq_n, b.err);
                 }
             }
@@ -1004,7 +1006,7 @@ cudaError_t launch_density(const DevParams& P, const StepBuffers& b, cudaStream_
                 if (e != cudaSuccess) return e;
                 auto k = b.sr.scenes ? k_density_geo<true> : k_density_geo<false>;
                 k<<<geo_grid(k, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, b.table, b.order, b.bcount,
-                                                              b.boffset, b.keys_tmp, b.rr, b.nlist, b.ncount,
+                                                              b.boffset, b.keys_tmp, b.rr, b.records(), b.nlist, b.ncount,
                                                               b.scanq, b.scanq_n, b.err);
             }
     }
@@ -1028,13 +1030,18 @@ cudaError_t launch_force(const DevParams& P, const StepBuffers& b, cudaStream_t 
             // (the grid search has a queue of its own)
             const unsigned qb = b.all_geo ? 0u : g;
             // the fast form sums the listed terms with fused arithmetic
-            auto kf = b.sr.scenes ? (b.fast ? k_force_list<true, true> : k_force_list<true, false>)
-                                  : (b.fast ? k_force_list<false, true> : k_force_list<false, false>);
-            kf<<<qb + g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, b.rr, b.table, b.order, b.nlist,
+            auto form = [&](auto packed) {
+                constexpr bool R = decltype(packed)::value;
+                return b.sr.scenes ? (b.fast ? k_force_list<true, true, R> : k_force_list<true, false, R>)
+                                   : (b.fast ? k_force_list<false, true, R> : k_force_list<false, false, R>);
+            };
+            float4* const fr = b.records();
+            auto kf = fr ? form(std::true_type{}) : form(std::false_type{});
+            kf<<<qb + g, NBR_THREADS, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, b.rr, fr, b.table, b.order, b.nlist,
                                               b.ncount, b.scanq, b.scanq_n, qb, b.all_geo, b.v, b.err);
             if (b.geo_any) {
                 auto k = b.sr.scenes ? k_force_geo<true> : k_force_geo<false>;
-                k<<<geo_grid(k, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, b.rr, b.table, b.order,
+                k<<<geo_grid(k, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, b.vp, b.vs, b.rr, fr, b.table, b.order,
                                                               b.bcount, b.boffset, b.scanq, b.scanq_n, b.v, b.err);
             }
         }

@@ -25,7 +25,8 @@ constexpr int SMALL_THREADS = 128;
 template <class F>
 __global__ void __launch_bounds__(SMALL_THREADS)
 k_density_small(DevParams P, F form, const float4* __restrict__ xp, const int2* __restrict__ table,
-                uint32_t* __restrict__ order, float2* __restrict__ rr, int32_t* __restrict__ nlist,
+                uint32_t* __restrict__ order, float2* __restrict__ rr, float4* __restrict__ fr,
+                int32_t* __restrict__ nlist,
                 int32_t* __restrict__ ncount, uint32_t* __restrict__ scanq, uint32_t* __restrict__ scanq_n,
                 uint32_t* __restrict__ err) {
     const uint32_t full = 0xffffffffu, n = P.n;
@@ -106,7 +107,7 @@ k_density_small(DevParams P, F form, const float4* __restrict__ xp, const int2* 
     }
     if (lane == 0) {
         const bool scan = !(list_ok && cnt <= P.list_cap);
-        rr[i] = sum.finish(P);
+        put_rr(rr, fr, i, sum.finish(P));
         order[i] = i;
         ncount[i] = scan ? -1 : (int32_t)cnt;
         if (scan) {
@@ -119,7 +120,7 @@ k_density_small(DevParams P, F form, const float4* __restrict__ xp, const int2* 
 template <class F>
 cudaError_t launch_density_small(const DevParams& P, const StepBuffers& b, const F& form, cudaStream_t s) {
     const unsigned g = (P.n + SMALL_THREADS / 32 - 1) / (SMALL_THREADS / 32);
-    k_density_small<F><<<g, SMALL_THREADS, 0, s>>>(P, form, b.xp, b.table, b.order, b.rr, b.nlist, b.ncount, b.scanq,
+    k_density_small<F><<<g, SMALL_THREADS, 0, s>>>(P, form, b.xp, b.table, b.order, b.rr, b.records(), b.nlist, b.ncount, b.scanq,
                                                    b.scanq_n, b.err);
     return cudaGetLastError();
 }

@@ -344,7 +344,7 @@ k_density_staged(DevParams P, const float4* __restrict__ xp,
                  const int2* __restrict__ table, const uint32_t* __restrict__ order,
                  const uint32_t* __restrict__ bseg, const uint32_t* __restrict__ btot,
                  const uint32_t* __restrict__ blist, uint32_t* __restrict__ counters,
-                 float2* __restrict__ rr, int32_t* __restrict__ nlist,
+                 float2* __restrict__ rr, float4* __restrict__ fr, int32_t* __restrict__ nlist,
                  int32_t* __restrict__ ncount, uint32_t* __restrict__ scanq,
                  uint32_t* __restrict__ scanq_n, uint32_t* __restrict__ err) {
     extern __shared__ __align__(16) unsigned char st_smem[];
@@ -428,9 +428,9 @@ k_density_staged(DevParams P, const float4* __restrict__ xp,
             }
             if (walk) {
                 for (int e = 0; e < cd; e++) st_density_term<FAST>(S.dd[e][tid], h, m, tot, tot_n);
-                rr[i] = st_density_finish<FAST>(P, tot, tot_n);
+                put_rr(rr, fr, i, st_density_finish<FAST>(P, tot, tot_n));
             } else if (live) {
-                rr[i] = density_scan_one(P, sp, xp, table, err);
+                put_rr(rr, fr, i, density_scan_one(P, sp, xp, table, err));
             }
             // the force pass: a list, or its scan queue
             const bool scan = live && !(walk && nl <= cap);
@@ -487,13 +487,13 @@ cudaError_t launch_density_staged(const DevParams& P, const StepBuffers& b, bool
         auto k = k_density_staged<true>;
         if ((e = allow_smem(k, smem)) != cudaSuccess) return e;
         k<<<staged_grid(k, smem), ST_THREADS, smem, s>>>(P, b.xp, b.table, b.order, b.bseg, b.btot,
-                                                         b.blist, b.st_counters, b.rr, b.nlist,
+                                                         b.blist, b.st_counters, b.rr, b.records(), b.nlist,
                                                          b.ncount, b.scanq, b.scanq_n, b.err);
     } else {
         auto k = k_density_staged<false>;
         if ((e = allow_smem(k, smem)) != cudaSuccess) return e;
         k<<<staged_grid(k, smem), ST_THREADS, smem, s>>>(P, b.xp, b.table, b.order, b.bseg, b.btot,
-                                                         b.blist, b.st_counters, b.rr, b.nlist,
+                                                         b.blist, b.st_counters, b.rr, b.records(), b.nlist,
                                                          b.ncount, b.scanq, b.scanq_n, b.err);
     }
     return cudaGetLastError();

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(ELEM_THREADS)
 k_reorder(DevParams P0, SceneRef sr, const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ perm,
           const float4* __restrict__ x, const float4* __restrict__ v,
           const uint32_t* __restrict__ ids, float4* __restrict__ xs, float4* __restrict__ vs,
-          float4* __restrict__ xp, float4* __restrict__ vp, uint32_t* __restrict__ ids_s,
+          float4* __restrict__ xp, float4* __restrict__ vp, float4* __restrict__ fr, uint32_t* __restrict__ ids_s,
           int2* __restrict__ table, uint32_t* __restrict__ bucket, uint32_t* __restrict__ brank,
           uint32_t* __restrict__ bcount, uint32_t* __restrict__ bcounter,
           uint32_t* __restrict__ scanq_n, uint4* __restrict__ rec, uint32_t* __restrict__ st_counters,
@@ -87,6 +87,10 @@ k_reorder(DevParams P0, SceneRef sr, const uint32_t* __restrict__ skeys, const u
     euler_walls(P, P.margin_p, pos, vel);
     xp[s] = make_float4(pos.x, pos.y, pos.z, 1.0f);
     vp[s] = make_float4(vel.x, vel.y, vel.z, 1.0f);
+    if (fr) {
+        fr[2 * (size_t)s] = make_float4(pos.x, pos.y, pos.z, vo.x);
+        fr[2 * (size_t)s + 1] = make_float4(vo.y, vo.z, 0.0f, 0.0f);
+    }
     if (rec) rec[s] = make_record(P, pos, vo);  // FP16-cell form
     // block of x* for the neighbour passes' processing order (any order gives
     // the same results; this one keeps a warp's neighbours in cache)
@@ -257,12 +261,12 @@ cudaError_t launch_reorder(const DevParams& P, const StepBuffers& b, cudaStream_
     uint32_t* bcount = ordered ? b.bcount : nullptr;
     if (b.sr.scenes)
         k_reorder<true><<<g, ELEM_THREADS, 0, s>>>(P, b.sr, b.skeys, b.perm, b.x, b.v, b.ids, b.xs,
-                                                   b.vs, b.xp, b.vp, b.ids_s, b.table, b.bucket,
+                                                   b.vs, b.xp, b.vp, b.records(), b.ids_s, b.table, b.bucket,
                                                    b.brank, bcount, b.bcounter, b.scanq_n, b.rec,
                                                    b.st_counters, b.err);
     else
         k_reorder<false><<<g, ELEM_THREADS, 0, s>>>(P, b.sr, b.skeys, b.perm, b.x, b.v, b.ids, b.xs,
-                                                    b.vs, b.xp, b.vp, b.ids_s, b.table, b.bucket,
+                                                    b.vs, b.xp, b.vp, b.records(), b.ids_s, b.table, b.bucket,
                                                     b.brank, bcount, b.bcounter, b.scanq_n, b.rec,
                                                     b.st_counters, b.err);
     if (!ordered) return cudaGetLastError();

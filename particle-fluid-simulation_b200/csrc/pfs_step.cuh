@@ -19,6 +19,17 @@ struct StepBuffers {
     float4* xp;         // predicted positions x*
     float4* vp;         // predicted velocities v*
     float2* rr;         // (density, near density)
+    // FP32 form of a table that grid search serves (may be null): what the force
+    // pass reads of a neighbour, 32 bytes (x* y* z* v.x | v.y v.z density near);
+    // the reorder writes the first six, the density pass the last two (put_rr)
+    float4* fr;
+    // Used where every particle is the grid search's: a few table slots mean
+    // hundreds of neighbours per particle, read as one aligned sector each in
+    // place of three parts (300,000 dense particles: force pass 960 -> 815 us for
+    // 1 us more in the reorder).  With a full table's tens of neighbours the
+    // record costs what it gives: 1,000,000-particle slab 157 -> 149 us and 9 us
+    // more in the reorder; 4,194,304 particles 434 -> 432 and 55 us more.
+    float4* records() const { return all_geo ? fr : nullptr; }
     uint32_t* keys;     // keys of the state positions (next sort's input)
     uint32_t* skeys;    // sorted keys
     uint32_t* perm;     // sort permutation

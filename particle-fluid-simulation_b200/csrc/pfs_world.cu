@@ -236,7 +236,7 @@ void* Arena::take(size_t n) {
 }
 
 size_t world_arena_bytes(uint32_t n, int flags, int precision, uint32_t blocks, uint32_t list_cap,
-                         uint32_t staged_blocks) {
+                         uint32_t staged_blocks, bool records) {
     const size_t f4 = (size_t)n * 16, u = (size_t)n * 4;
     size_t b = u /*clist*/ + 6 * f4 /*x v xs vs xp vp*/ + (size_t)n * 8 /*rr*/ + 5 * u /*keys skeys perm tmp x2*/ +
                sort_scratch_words(n, sort_key_bits(n)) * 4 + (size_t)n * 8 /*table*/ + 256 /*err*/ +
@@ -246,6 +246,7 @@ size_t world_arena_bytes(uint32_t n, int flags, int precision, uint32_t blocks, 
     if (flags & PFS_FLAG_IDS_INTERNAL) b += 2 * u;
     if (flags & PFS_FLAG_COLORS) b += f4;
     if (precision == PFS_FP16_CELL) b += fp16_arena_bytes(n);
+    if (records) b += 2 * f4 /*fr*/;
     return b + 32 * 256;  // alignment slack
 }
 
@@ -401,8 +402,9 @@ int carve(pfs_world* w) {
     uint32_t blocks = spatial_blocks(w->dp);
     if (w->staged_ok) blocks = std::max<uint32_t>(blocks, (uint32_t)staged_buckets(w->staged_cfg));
     w->blocks_cap = blocks;
+    const bool records = w->params.precision != PFS_FP16_CELL && w->dp.geo != 0;
     cudaError_t e = a.reserve(world_arena_bytes(n, w->flags, w->params.precision, blocks, w->list_cap,
-                                                w->staged_blocks));
+                                                w->staged_blocks, records));
     if (e != cudaSuccess) return status_from_cuda(e);
     const size_t f4 = (size_t)n * 16, u = (size_t)n * 4;
     StepBuffers& b = w->b;
@@ -413,6 +415,7 @@ int carve(pfs_world* w) {
     b.xp = (float4*)a.take(f4);
     b.vp = (float4*)a.take(f4);
     b.rr = (float2*)a.take((size_t)n * 8);
+    b.fr = records ? (float4*)a.take(2 * f4) : nullptr;
     b.keys = (uint32_t*)a.take(u);
     b.skeys = (uint32_t*)a.take(u);
     b.perm = (uint32_t*)a.take(u);
@@ -459,7 +462,8 @@ int carve(pfs_world* w) {
         if (!fp16_carve(a, n, &w->h16)) return PFS_ENOMEM;
     }
     if (!b.x || !b.v || !b.xs || !b.vs || !b.xp || !b.vp || !b.rr || !b.keys || !b.skeys ||
-        !b.perm || !b.keys_tmp || !b.vals_tmp || !b.sort_scratch || !b.table || !b.err)
+        !b.perm || !b.keys_tmp || !b.vals_tmp || !b.sort_scratch || !b.table || !b.err ||
+        (records && !b.fr))
         return PFS_ENOMEM;
     w->err = b.err;
     return PFS_OK;

@@ -94,3 +94,24 @@ def test_cells_pairs_on_the_cut(cuda_device, seed):
             assert w.device_error() == 0
     for k in ("density", "near_density", "vel_force"):
         _assert_bits_equal(k, out[pfs.PFS_SEARCH_GRID][k], out[pfs.PFS_SEARCH_TABLE][k])
+
+
+@pytest.mark.parametrize("fast", [False, True])
+@pytest.mark.parametrize("n", [33, 12289])
+def test_force_records_change_nothing(cuda_device, monkeypatch, n, fast):
+    """The force pass reads a neighbour as one 32-byte record in a world created for
+    the grid search, as three parts in one that comes to it later: the same bits."""
+    pfs = load_package()
+    p, pos, vel = _uniform_scene(pfs, n, seed=n, h=0.12)
+    if fast:
+        p.precision = pfs.PFS_FP32_FAST
+    out = {}
+    for mode in ("table", "grid"):
+        monkeypatch.setenv("PFS_NEIGHBOR_SEARCH", mode)
+        with pfs.World(p, pos, vel) as w:
+            w.set_shape(pfs.PFS_SHAPE_FLAT, pfs.PFS_SEARCH_GRID)
+            w.step(2)
+            out[mode] = w.read(pos=True, vel=True, density=True)
+            assert w.device_error() == 0
+    for k in ("pos", "vel", "density"):
+        _assert_bits_equal(k, out["grid"][k], out["table"][k])
