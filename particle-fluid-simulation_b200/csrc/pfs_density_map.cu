@@ -12,7 +12,8 @@
 // is rebuilt from its sorted keys for the call (the step's integrate clears it)
 // and cleared again.
 //
-// The work is grouped by cell (k_map_cells), as in the density pass of the grid
+// Where the table has few slots the work is grouped by cell (k_map_cells; elsewhere
+// k_map_flat), as in the density pass of the grid
 // search (pfs_cells.cuh).  One thread per voxel walking its own 27 runs waits on
 // 27 table look-ups, and reads, where the table has few slots, hundreds of
 // distant particles per run: 5.2 ms for the reference's 300,000 particles (4,096
@@ -29,6 +30,7 @@
 
 #include "pfs_cells.cuh"
 #include "pfs_common.cuh"
+#include "pfs_flat.cuh"
 #include "pfs_step.cuh"
 
 namespace pfs {
@@ -127,10 +129,10 @@ __device__ float map_walk(const DevParams& P, const MapArgs& A, float cxp, float
     return PFS_DIV(PFS_MUL(density, 1.0f), P.volume);
 }
 
-// The voxels the shader skips (0), and the rest of those whose centre lies
-// outside the box, or with `all` every voxel.
+// Beside the cells' pass: the voxels the shader skips (0), and the rest of those
+// whose centre lies outside the box.
 __global__ void __launch_bounds__(MAP_THREADS)
-k_density_map(DevParams P, MapArgs A, uint32_t all, const float4* __restrict__ x, const int2* __restrict__ table,
+k_density_map(DevParams P, MapArgs A, const float4* __restrict__ x, const int2* __restrict__ table,
               float* __restrict__ out, uint32_t* __restrict__ err) {
     const uint64_t nx = (uint64_t)A.img.x, ny = (uint64_t)A.img.y, nz = (uint64_t)A.img.z;
     const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -141,7 +143,130 @@ k_density_map(DevParams P, MapArgs A, uint32_t all, const float4* __restrict__ x
         return;
     }
     const float cx = map_centre(P.minx, vx, A.cs), cy = map_centre(P.miny, vy, A.cs), cz = map_centre(P.minz, vz, A.cs);
-    if (all || !map_inside(P, cx, cy, cz)) out[idx] = map_walk(P, A, cx, cy, cz, x, table, err);
+    if (!map_inside(P, cx, cy, cz)) out[idx] = map_walk(P, A, cx, cy, cz, x, table, err);
+}
+
+// Every voxel, by the flat walk of pfs_flat.cuh (a thread per voxel, the voxels of
+// a block sorted by their candidate totals, one loop over the 27 runs together).
+// A loop per run ran with 12 of 32 lanes: neighbouring voxels' runs differ in
+// length, their totals little.  1,000,000 voxels of a 1,048,576-particle slab:
+// 310 -> 250 us (now the L1 binds it: a lane's candidate is a line of its own).
+// Voxels with more than FLAT_RCAP run words walk by themselves.
+__global__ void __launch_bounds__(FLAT_THREADS, FLAT_BLOCKS)
+k_map_flat(DevParams P, MapArgs A, const float4* __restrict__ x, const int2* __restrict__ table,
+           float* __restrict__ out, uint32_t* __restrict__ err) {
+    __shared__ FlatShared S;
+    __shared__ float s_dd[FLAT_CAP][FLAT_THREADS];  // per thread: deferred terms
+    const int tid = threadIdx.x;
+    const uint32_t n = P.n;
+    const uint64_t nx = (uint64_t)A.img.x, ny = (uint64_t)A.img.y, nz = (uint64_t)A.img.z;
+    const uint64_t first = (uint64_t)blockIdx.x * FLAT_THREADS;
+    __shared__ uint32_t s_first[3];  // the block's first voxel
+    if (tid == 0) {
+        s_first[0] = (uint32_t)(first % nx);
+        s_first[1] = (uint32_t)((first / nx) % ny);
+        s_first[2] = (uint32_t)(first / (nx * ny));
+    }
+    __syncthreads();
+    auto voxel = [&](int col, float& cx, float& cy, float& cz) {  // false: none, or one the shader skips
+        const uint64_t idx = first + (uint64_t)col;
+        const uint32_t ix = s_first[0] + (uint32_t)col, iy = s_first[1] + ix / (uint32_t)nx;
+        const int32_t vx = (int32_t)(ix % (uint32_t)nx), vy = (int32_t)(iy % (uint32_t)ny),
+                      vz = (int32_t)(s_first[2] + iy / (uint32_t)ny);
+        cx = map_centre(P.minx, vx, A.cs);
+        cy = map_centre(P.miny, vy, A.cs);
+        cz = map_centre(P.minz, vz, A.cs);
+        return idx < nx * ny * nz && !map_out(vx, vy, vz, A.bound);
+    };
+    float cx, cy, cz;
+    const bool mine = voxel(tid, cx, cy, cz);
+    int nr = 0;
+    uint32_t tot = 0;
+    if (mine) {
+        int32_t c0 = -1, c1 = -1, c2 = -1;
+        if (map_inside(P, cx, cy, cz)) {
+            c0 = cell_coord(cx, P.minx, P.h);
+            c1 = cell_coord(cy, P.miny, P.h);
+            c2 = cell_coord(cz, P.minz, P.h);
+        }
+        // map_out of the 27 cells by axis
+        uint32_t hx[3], hy[3];
+        bool ox[3], oy[3], ex[3], ey[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const int32_t kx = c0 + a - 1, ky = c1 + a - 1;
+            hx[a] = (uint32_t)kx * 73856093u;
+            hy[a] = (uint32_t)ky * 19349663u;
+            ox[a] = kx < 0 || kx > A.bound.x;
+            oy[a] = ky < 0 || ky > A.bound.y;
+            ex[a] = kx == A.bound.x;
+            ey[a] = ky == A.bound.y;
+        }
+#pragma unroll 1
+        for (int dz = -1; dz <= 1; dz++) {
+            const int32_t kz = c2 + dz;
+            if (kz < 0 || kz > A.bound.z) continue;
+            const uint32_t hz = (uint32_t)kz * 83492791u;
+            const bool ez = kz == A.bound.z;
+            // a layer's nine table entries are loaded together
+            int2 row[9];
+#pragma unroll
+            for (int q = 0; q < 9; q++)
+                row[q] = ox[q % 3] || oy[q / 3] || (ex[q % 3] && ey[q / 3] && ez)
+                             ? make_int2(-1, -1)
+                             : __ldg(table + slot_of(P, hash_finalize(hx[q % 3] ^ hy[q / 3] ^ hz)));
+#pragma unroll
+            for (int q = 0; q < 9; q++) {
+                const int2 se = row[q];
+                if (se.x == -1) continue;
+                if (se.x < 0 || se.y > (int32_t)n || se.x > se.y) {
+                    atomicOr(err, ERR_TABLE_RANGE);
+                    continue;
+                }
+                uint32_t s0 = (uint32_t)se.x, len = (uint32_t)(se.y - se.x);
+                tot += len;
+                while (len > 0) {
+                    const uint32_t l = min(len, FLAT_LEN_MAX);
+                    if (nr < FLAT_RCAP) S.rng[nr][tid] = s0 | (l << 24);
+                    nr++;
+                    s0 += l;
+                    len -= l;
+                }
+            }
+        }
+    }
+    const bool own = nr > FLAT_RCAP;
+    if (nr == 0 || own) S.rng[0][tid] = 0u;  // an empty walk
+    S.meta[tid] = (uint8_t)(own ? FLAT_OVER : 0u);
+    const uint32_t key = flat_sort(((own ? 0u : tot) << 7) | (uint32_t)tid, reinterpret_cast<uint32_t*>(&s_dd[0][0]), S);
+    const int src = (int)(key & 127u);
+    const uint32_t meta = S.meta[src];
+    flat_move(src, S);
+    const bool live = voxel(src, cx, cy, cz);
+    float density = 0.0f;
+    float* dp = &s_dd[0][tid];
+    float* const dfull = &s_dd[FLAT_CAP - 1][tid];
+    auto test = [&](const float4 p, int32_t, bool, bool valid) {
+        const float d0 = PFS_SUB(cx, p.x), d1 = PFS_SUB(cy, p.y), d2 = PFS_SUB(cz, p.z);
+        const float dist2 = PFS_ADD(PFS_ADD(PFS_MUL(d0, d0), PFS_MUL(d1, d1)), PFS_MUL(d2, d2));
+        *dp = dist2;
+        dp += (valid && dist2 < P.r2) ? FLAT_THREADS : 0;
+    };
+    auto drain_if_full = [&]() {
+        if (__any_sync(0xffffffffu, dp >= dfull)) {
+            for (int c = 0; c < FLAT_CAP; c++)
+                if (&s_dd[c][tid] < dp) density = PFS_ADD(density, map_term(P, s_dd[c][tid]));
+            dp = &s_dd[0][tid];
+        }
+    };
+    flat_walk(S, (int32_t)(key >> 7), 0, true, [&](int32_t j) { return __ldg(x + j); }, test, drain_if_full);
+    for (const float* e = &s_dd[0][tid]; e < dp; e += FLAT_THREADS) density = PFS_ADD(density, map_term(P, *e));
+    const uint64_t idx = first + (uint64_t)src;
+    if (live)
+        out[idx] = (meta & FLAT_OVER) ? map_walk(P, A, cx, cy, cz, x, table, err)
+                                      : PFS_DIV(PFS_MUL(density, 1.0f), P.volume);
+    else if (idx < nx * ny * nz)
+        out[idx] = 0.0f;
 }
 
 // Voxels per warp up to which it evaluates terms as it tests: about 50 instructions
@@ -645,8 +770,8 @@ cudaError_t launch_density_map(const DevParams& P, const StepBuffers& b, float c
         const unsigned gv = (unsigned)((voxels + MAP_THREADS - 1) / MAP_THREADS);
         DevParams M = P;
         map_blocks(&M, cell_size, per_cell);
-        // Where runs hold a few entries the voxels' own walks are as fast (1M-particle
-        // slab, full table, 1M voxels: 0.32 ms against 0.38), so the blocks take over
+        // Where runs hold a few entries the voxels' own walks are faster (1M-particle
+        // slab, full table, 1M voxels: 0.25 ms against 0.38), so the blocks take over
         // where the grid search does.
         // (a grid of many more cells than voxels has little to group, and the list of
         // blocks takes a sort buffer)
@@ -654,8 +779,13 @@ cudaError_t launch_density_map(const DevParams& P, const StepBuffers& b, float c
         const bool cells = (n >> __builtin_popcount(P.mask)) >= 4u &&
                            std::max(P.ngx, std::max(P.ngy, P.ngz)) <= CELLS_MAX_GRID &&
                            blocks <= (double)std::min<uint64_t>(voxels, n);
-        k_density_map<<<gv, MAP_THREADS, 0, s>>>(P, A, cells ? 0u : 1u, b.x, b.table, out, b.err);
-        if (cells) {
+        if (!cells) {
+            const cudaError_t e = flat_carveout(k_map_flat);
+            if (e != cudaSuccess) return e;
+            const unsigned gf = (unsigned)((voxels + FLAT_THREADS - 1) / FLAT_THREADS);
+            k_map_flat<<<gf, FLAT_THREADS, 0, s>>>(P, A, b.x, b.table, out, b.err);
+        } else {
+            k_density_map<<<gv, MAP_THREADS, 0, s>>>(P, A, b.x, b.table, out, b.err);
             k_map_code<<<g, MAP_THREADS, 0, s>>>(P, b.x, b.keys_tmp);
             const CellsLayout lay = {MAP_STAGE, 256u, 20u};
             const size_t dyn = (size_t)lay.entries * 16 + CELLS_WARPS * (size_t)cells_warp_bytes(lay);
