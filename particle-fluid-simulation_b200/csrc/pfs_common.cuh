@@ -273,4 +273,13 @@ __device__ __forceinline__ void put_rr(float2* __restrict__ rr, float4* __restri
     if (fr) *(reinterpret_cast<float2*>(fr) + 4 * (size_t)i + 3) = d;
 }
 
+// a / b given y = RN(1 / b), by Markstein's correction (P. Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", 1990): the
+// residual of RN(a y) is exact in one fused operation, and the corrected quotient
+// is the correctly rounded one, as long as nothing underflows or overflows.
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+    const float q = PFS_MUL(a, y);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+
 }  // namespace pfs

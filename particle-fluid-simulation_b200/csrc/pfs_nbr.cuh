@@ -179,15 +179,6 @@ __device__ __forceinline__ void force_term(const DevParams& P, const ForceSelf& 
     force_term_pre(P, me, __ldg(xp + j), __ldg(rr + j), __ldg(vs + j), f);
 }
 
-// a / b given y = RN(1 / b), by Markstein's correction (P. Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000 processor", 1990): the
-// residual of RN(a y) is exact in one fused operation, and the corrected quotient
-// is the correctly rounded one, as long as nothing underflows or overflows.
-__device__ __forceinline__ float div_by(float a, float b, float y) {
-    const float q = PFS_MUL(a, y);
-    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
-}
-
 // The five quotients of a neighbour's force terms: its direction d / dist, and
 // the pressure and viscosity coefficients c / dj and v / dj (dj >= 0.01).  Two
 // reciprocals serve all five; a third of the pass's instructions were the
