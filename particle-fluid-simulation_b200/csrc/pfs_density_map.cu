@@ -63,17 +63,45 @@ k_table_runs(uint32_t n, const uint32_t* __restrict__ skeys, int2* __restrict__ 
     if (tail) table[k].y = (int32_t)(s + 1);
 }
 
-// Packed positions of the state (bits as cells_code; NaN is marked in bit 31).
+// Packed positions of the state (bits as cells_code; NaN is marked in bit 31).  Each
+// position marks its cell (marks: a byte per cell of the grid padded to whole
+// blocks of 4 x 4 x 4) and, for rounding, those a sixteenth away: a cell coordinate
+// is below CELLS_MAX_GRID and good to 2^-6.
 __global__ void __launch_bounds__(MAP_THREADS)
-k_map_code(DevParams P, const float4* __restrict__ x, uint32_t* __restrict__ code) {
+k_map_code(DevParams P, const float4* __restrict__ x, uint32_t* __restrict__ code, uint8_t* __restrict__ marks) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.n) return;
-    const float4 p = x[i];
+    const bool live = i < P.n;
+    const float4 p = live ? x[i] : make_float4(NAN, NAN, NAN, 0.0f);
     const float s = (float)CELLS_CODE_STEPS;
-    auto field = [&](float v, float mn) { return (uint32_t)__float2int_rd(PFS_DIV(PFS_SUB(v, mn), P.h) * s) & 511u; };
+    const float u[3] = {PFS_DIV(PFS_SUB(p.x, P.minx), P.h), PFS_DIV(PFS_SUB(p.y, P.miny), P.h),
+                        PFS_DIV(PFS_SUB(p.z, P.minz), P.h)};
+    const uint32_t g[3] = {(P.ngx & ~3u) + 4, (P.ngy & ~3u) + 4, (P.ngz & ~3u) + 4};
+    auto field = [&](float v) { return (uint32_t)__float2int_rd(v * s) & 511u; };
     const bool nan = isnan(p.x) || isnan(p.y) || isnan(p.z);
-    code[i] = field(p.x, P.minx) | field(p.y, P.miny) << 10 | field(p.z, P.minz) << 20 | CELLS_GUARD |
-              (nan ? 0x80000000u : 0u);
+    if (live) code[i] = field(u[0]) | field(u[1]) << 10 | field(u[2]) << 20 | CELLS_GUARD | (nan ? 0x80000000u : 0u);
+    int lo[3], hi[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const bool near = u[a] > -2.0f && u[a] < (float)g[a] + 2.0f;  // elsewhere nothing reaches the box
+        lo[a] = near ? max(__float2int_rd(u[a] - 0.0625f), 0) : 0;
+        hi[a] = near ? min(__float2int_rd(u[a] + 0.0625f), (int)g[a] - 1) : -1;
+        if (near && hi[a] < 0) hi[a] = 0;                             // a cell outside marks the
+        if (near && lo[a] >= (int)g[a]) lo[a] = (int)g[a] - 1;        // nearest inside
+    }
+    // the positions of a table run come from few cells: one lane marks for all that
+    // mark the same (every lane for itself: 46 us for 300,000 particles; so: 35)
+    const bool marks_any = lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2];
+    const unsigned long long same =
+        !marks_any ? ~0ull
+                   : (unsigned long long)lo[0] | (unsigned long long)lo[1] << 17 | (unsigned long long)lo[2] << 34 |
+                         (unsigned long long)((hi[0] - lo[0]) | (hi[1] - lo[1]) << 1 | (hi[2] - lo[2]) << 2) << 51;
+    if ((int)(threadIdx.x & 31) != __ffs(__match_any_sync(0xffffffffu, same)) - 1) return;
+    for (int z = lo[2]; z <= hi[2]; z++)
+        for (int y = lo[1]; y <= hi[1]; y++)
+            for (int q = lo[0]; q <= hi[0]; q++) {
+                uint8_t* m = marks + ((size_t)q + (size_t)g[0] * ((size_t)y + (size_t)g[1] * (size_t)z));
+                if (__ldcg(m) == 0u) __stcg(m, (uint8_t)1);
+            }
 }
 
 struct MapArgs {
@@ -411,46 +439,48 @@ __device__ __forceinline__ void map_first(const DevParams& P, const MapArgs& A, 
     first[a][k] = v;
 }
 
-// Most of a box is empty: blocks of 4 x 4 x 4 cells with nothing near them are
-// set to 0 here, and only the blocks (nbx x nby x nbz of 2^bs cells) of the others
-// are listed for k_map_cells.
-__global__ void __launch_bounds__(CELLS_THREADS, 5)
-k_map_coarse(DevParams P, MapArgs A, CellsLayout lay, const float4* __restrict__ x, const int2* __restrict__ table,
-             const uint32_t* __restrict__ code, float* __restrict__ out, uint32_t* __restrict__ list,
-             uint32_t* __restrict__ listed, uint32_t* __restrict__ err) {
-    extern __shared__ float4 s_dyn[];
-    __shared__ MapShared S;
+// Most of a box is empty: blocks of 4 x 4 x 4 cells with no marked cell in them or
+// next to them are set to 0 here, and only the blocks (nbx x nby x nbz of 2^bs cells)
+// of the others are listed for k_map_cells.  (Finding the empty ones by scanning
+// the 216 runs around each, which in a table of few slots hold hundreds of distant
+// positions, took 133 us of a 300,000-particle scene's map; marking takes 31 and this 11.)
+__global__ void __launch_bounds__(CELLS_THREADS)
+k_map_coarse(DevParams P, MapArgs A, const uint8_t* __restrict__ marks, float* __restrict__ out,
+             uint32_t* __restrict__ list, uint32_t* __restrict__ listed) {
+    __shared__ int32_t s_first[3][8];
     const int tid = threadIdx.x;
-    uint32_t* zone =
-        reinterpret_cast<uint32_t*>(s_dyn + lay.entries) + (tid >> 5) * (cells_warp_bytes(lay) / 4);
-    const uint32_t gx = (P.ngx >> 2) + 1, gy = (P.ngy >> 2) + 1, gz = (P.ngz >> 2) + 1;
-    const int3 dim = make_int3(4, 4, 4);
-    for (uint32_t blk = blockIdx.x; blk < gx * gy * gz; blk += gridDim.x) {
-        const int3 b = make_int3((int)(blk % gx) << 2, (int)(blk / gx % gy) << 2, (int)(blk / (gx * gy)) << 2);
-        const bool fits = map_build(P, A, S, lay, s_dyn, zone, b, dim, 0, 6, x, table, code, err);
-        if (!fits || S.off[216] != 0u) {
-            const uint32_t fx = 4u >> P.bsx, fy = 4u >> P.bsy, fz = 4u >> P.bsz;
-            const uint32_t k = tid;
-            if (k < fx * fy * fz) {
-                const uint32_t qx = ((uint32_t)b.x >> P.bsx) + k % fx, qy = ((uint32_t)b.y >> P.bsy) + k / fx % fy,
-                               qz = ((uint32_t)b.z >> P.bsz) + k / (fx * fy);
-                if (qx < P.nbx && qy < P.nby && qz < P.nbz)
-                    list[atomicAdd(listed, 1u)] = qx + P.nbx * (qy + P.nby * qz);
-            }
-            continue;
+    const uint32_t gx = (P.ngx >> 2) + 1, gy = (P.ngy >> 2) + 1;
+    const uint32_t blk = blockIdx.x;
+    const int3 b = make_int3((int)(blk % gx) << 2, (int)(blk / gx % gy) << 2, (int)(blk / (gx * gy)) << 2);
+    const int3 g = make_int3((int)gx << 2, (int)gy << 2, (int)((P.ngz >> 2) + 1) << 2);
+    bool any = false;
+    for (int r = tid; r < 216; r += CELLS_THREADS) {
+        const int cx = b.x - 1 + r % 6, cy = b.y - 1 + r / 6 % 6, cz = b.z - 1 + r / 36;
+        if (cx >= 0 && cy >= 0 && cz >= 0 && cx < g.x && cy < g.y && cz < g.z)
+            any = any || marks[(size_t)cx + (size_t)g.x * ((size_t)cy + (size_t)g.y * (size_t)cz)] != 0;
+    }
+    if (__syncthreads_or(any)) {
+        const uint32_t fx = 4u >> P.bsx, fy = 4u >> P.bsy, fz = 4u >> P.bsz;
+        const uint32_t k = tid;
+        if (k < fx * fy * fz) {
+            const uint32_t qx = ((uint32_t)b.x >> P.bsx) + k % fx, qy = ((uint32_t)b.y >> P.bsy) + k / fx % fy,
+                           qz = ((uint32_t)b.z >> P.bsz) + k / (fx * fy);
+            if (qx < P.nbx && qy < P.nby && qz < P.nbz)
+                list[atomicAdd(listed, 1u)] = qx + P.nbx * (qy + P.nby * qz);
         }
-        map_first(P, A, b, S.first);
-        __syncthreads();
-        const int wx = S.first[0][4] - S.first[0][0], wy = S.first[1][4] - S.first[1][0],
-                  wz = S.first[2][4] - S.first[2][0];
-        for (int k = tid; k < wx * wy * wz; k += CELLS_THREADS) {
-            const int vx = S.first[0][0] + k % wx, vy = S.first[1][0] + k / wx % wy, vz = S.first[2][0] + k / (wx * wy);
-            if (map_out(vx, vy, vz, A.bound) ||
-                !map_inside(P, map_centre(P.minx, vx, A.cs), map_centre(P.miny, vy, A.cs), map_centre(P.minz, vz, A.cs)))
-                continue;  // k_density_map's
-            out[((uint64_t)vz * (uint64_t)A.img.y + (uint64_t)vy) * (uint64_t)A.img.x + (uint64_t)vx] =
-                PFS_DIV(0.0f, P.volume);
-        }
+        return;
+    }
+    map_first(P, A, b, s_first);
+    __syncthreads();
+    const int wx = s_first[0][4] - s_first[0][0], wy = s_first[1][4] - s_first[1][0],
+              wz = s_first[2][4] - s_first[2][0];
+    for (int k = tid; k < wx * wy * wz; k += CELLS_THREADS) {
+        const int vx = s_first[0][0] + k % wx, vy = s_first[1][0] + k / wx % wy, vz = s_first[2][0] + k / (wx * wy);
+        if (map_out(vx, vy, vz, A.bound) ||
+            !map_inside(P, map_centre(P.minx, vx, A.cs), map_centre(P.miny, vy, A.cs), map_centre(P.minz, vz, A.cs)))
+            continue;  // k_density_map's
+        out[((uint64_t)vz * (uint64_t)A.img.y + (uint64_t)vy) * (uint64_t)A.img.x + (uint64_t)vx] =
+            PFS_DIV(0.0f, P.volume);
     }
 }
 
@@ -786,18 +816,21 @@ cudaError_t launch_density_map(const DevParams& P, const StepBuffers& b, float c
             k_map_flat<<<gf, FLAT_THREADS, 0, s>>>(P, A, b.x, b.table, out, b.err);
         } else {
             k_density_map<<<gv, MAP_THREADS, 0, s>>>(P, A, b.x, b.table, out, b.err);
-            k_map_code<<<g, MAP_THREADS, 0, s>>>(P, b.x, b.keys_tmp);
+            // the marks take the neighbour lists' buffer (64 bytes for each 4 x 4 x 4 cells,
+            // of which there are at most n)
+            const uint32_t coarse = ((P.ngx >> 2) + 1) * ((P.ngy >> 2) + 1) * ((P.ngz >> 2) + 1);
+            static_assert(NLIST_CAP * 4 >= 64, "marks in the neighbour lists");
+            uint8_t* marks = reinterpret_cast<uint8_t*>(b.nlist);
+            cudaError_t e = cudaMemsetAsync(marks, 0, (size_t)coarse * 64, s);
+            if (e != cudaSuccess) return e;
+            k_map_code<<<g, MAP_THREADS, 0, s>>>(P, b.x, b.keys_tmp, marks);
             const CellsLayout lay = {MAP_STAGE, 256u, 20u};
             const size_t dyn = (size_t)lay.entries * 16 + CELLS_WARPS * (size_t)cells_warp_bytes(lay);
-            cudaError_t e = cudaFuncSetAttribute(k_map_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_map_coarse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+            e = cudaFuncSetAttribute(k_map_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
             uint32_t* listed = b.scanq_n + CTR_BLOCKS;
             if (e == cudaSuccess) e = cudaMemsetAsync(listed, 0, 4, s);
             if (e != cudaSuccess) return e;
-            const uint32_t coarse = ((P.ngx >> 2) + 1) * ((P.ngy >> 2) + 1) * ((P.ngz >> 2) + 1);
-            k_map_coarse<<<std::min(cells_grid(k_map_coarse, dyn), coarse), CELLS_THREADS, dyn, s>>>(
-                M, A, lay, b.x, b.table, b.keys_tmp, out, b.vals_tmp, listed, b.err);
+            k_map_coarse<<<coarse, CELLS_THREADS, 0, s>>>(M, A, marks, out, b.vals_tmp, listed);
             k_map_cells<<<std::min(cells_grid(k_map_cells, dyn), M.nbx * M.nby * M.nbz), CELLS_THREADS, dyn, s>>>(
                 M, A, lay, b.x, b.table, b.keys_tmp, b.vals_tmp, listed, out, b.err);
         }

@@ -41,3 +41,31 @@ def test_map_cells_match_oracle(cuda_device, n, h, factor, clump):
     want = ora.density_map(p, st["pos"], st["keys"], cs)
     assert np.count_nonzero(want) > 0
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("shift", [-0.0625, 0.0, 0.0625])
+def test_map_cells_between_empty_blocks(cuda_device, shift):
+    """Small clumps at the faces and corners of blocks of 4 x 4 x 4 cells (within
+    rounding of them and a step away) among empty blocks, and at the box's walls."""
+    pfs, ora = load_package(), load_oracle()
+    h, n = 0.06, 7937  # 32 slots
+    p, pos, vel = _uniform_scene(pfs, n, seed=5, h=h)
+    p.gravity[:] = (0.0, 0.0, 0.0)
+    lo, hi = np.array(p.box_min[:]), np.array(p.box_max[:])
+    rng = np.random.default_rng(9)
+    faces = np.arange(0, int((hi - lo).min() / h), 4)
+    spot = lo + h * (rng.choice(faces, (16, 3)) + shift)
+    spot[::2] += h * rng.integers(0, 5, (8, 3))
+    at = rng.integers(0, 16, n)
+    jitter = rng.choice([0.0, 1e-7, -1e-7, 0.01 * h, -0.01 * h], (n, 3))
+    pos[:, :3] = np.clip(spot[at] + jitter, lo + 1e-3, hi - 1e-3)
+    with pfs.World(p, pos, vel) as w:
+        w.step(1)
+        st = w.read(pos=True, keys=True)
+        for factor in (0.5, 1.0):
+            cs = float(np.float32(np.float32(h) * np.float32(factor)))
+            got = w.density_map(cs)
+            want = ora.density_map(p, st["pos"], st["keys"], cs)
+            assert 0 < np.count_nonzero(want) < want.size // 2
+            assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+        assert w.device_error() == 0
