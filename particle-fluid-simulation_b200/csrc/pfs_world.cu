@@ -618,15 +618,18 @@ const char* pfs_strerror(int s) {
 
 int pfs_version(void) { return 10000; }
 
-// Neighbour-list rows of a new world: twice the mean neighbour count of its
-// initial state (particles in their bounding box, clipped to the world box,
+// Neighbour-list rows of a new world: twice the mean neighbour count (with the grid
+// search eight times: there a particle without a list costs a gather by a whole
+// warp, and 150,000 dense particles that fall on each other spent 0.9 ms a substep
+// on them; elsewhere rows only cost memory, 9 ms of a 1,000,000-particle world's
+// creation) of its initial state (particles in their bounding box, clipped to the world box,
 // times the volume of a sphere of radius h), rounded up to 16 and kept within
 // [NLIST_CAP, NLIST_CAP_MAX].  Particles of denser regions than that fall back
 // to the force pass's scan, with the same results.
 static bool is_device_ptr(const void* p);
 static int apply_shape(pfs_world* w, int32_t shape, int32_t search);
 
-static uint32_t list_rows_for(const pfs_params& p, uint32_t n, const float* pos4) {
+static uint32_t list_rows_for(const pfs_params& p, uint32_t n, const float* pos4, bool geo) {
     if (n == 0 || !pos4) return NLIST_CAP;
     double lo[3], hi[3];
     for (int a = 0; a < 3; a++) {
@@ -653,7 +656,7 @@ static uint32_t list_rows_for(const pfs_params& p, uint32_t n, const float* pos4
     double vol = 1.0;
     for (int a = 0; a < 3; a++) vol *= std::max(hi[a] - lo[a], (double)p.h);
     const double h = p.h;
-    const double nb = 8.0 * (double)n / vol * (4.0 / 3.0) * 3.14159265358979 * h * h * h;
+    const double nb = (geo ? 8.0 : 2.0) * (double)n / vol * (4.0 / 3.0) * 3.14159265358979 * h * h * h;
     if (!(nb > NLIST_CAP)) return NLIST_CAP;
     if (nb >= NLIST_CAP_MAX) return NLIST_CAP_MAX;
     return std::min<uint32_t>(((uint32_t)nb + 15u) & ~15u, NLIST_CAP_MAX);
@@ -678,7 +681,7 @@ int pfs_world_create(const pfs_params* p, uint32_t n, const float* pos4, const f
     if (w->flags & PFS_FLAG_IDS) w->flags |= PFS_FLAG_IDS_INTERNAL;
     w->fluid = fluid_volume(*p, n, pos4);
     derive_params(*p, n, &w->dp, -1, w->fluid);
-    w->list_cap = list_rows_for(*p, n, pos4);
+    w->list_cap = list_rows_for(*p, n, pos4, w->dp.geo != 0);
     w->dp.list_cap = w->list_cap;
     {
         // staged block shape from the initial state's particles per cell
