@@ -29,6 +29,9 @@
 
 namespace pfs {
 
+// A table of a quarter as many slots as particles or fewer.
+static bool few_slots(uint32_t n) { return n >= 2 && (4ull << __builtin_popcount(n - 1u)) <= (uint64_t)n; }
+
 // Neighbour search of a table of n particles over a grid of g cells per
 // axis.  The table has 2^popcount(n - 1) slots; when that is a quarter of n
 // or less, slot ranges mix many distant cells and the grid search
@@ -42,9 +45,7 @@ static bool choose_grid_search(uint32_t n, const uint32_t g[3], int search) {
     const char* e = getenv("PFS_NEIGHBOR_SEARCH");
     if (e && strcmp(e, "table") == 0) return false;
     if (e && strcmp(e, "grid") == 0) return n > 0;
-    if (n < 2) return false;
-    const uint64_t slots = 1ull << __builtin_popcount(n - 1u);
-    return slots * 4 <= (uint64_t)n;
+    return few_slots(n);
 }
 
 static void set_block_counts(DevParams* o);
@@ -618,8 +619,8 @@ const char* pfs_strerror(int s) {
 
 int pfs_version(void) { return 10000; }
 
-// Neighbour-list rows of a new world: twice the mean neighbour count (with the grid
-// search eight times: there a particle without a list costs a gather by a whole
+// Neighbour-list rows of a new world: twice the mean neighbour count (eight times where
+// the table has few slots: there a particle without a list costs a gather by a whole
 // warp, and 150,000 dense particles that fall on each other spent 0.9 ms a substep
 // on them; elsewhere rows only cost memory, 9 ms of a 1,000,000-particle world's
 // creation) of its initial state (particles in their bounding box, clipped to the world box,
@@ -629,7 +630,7 @@ int pfs_version(void) { return 10000; }
 static bool is_device_ptr(const void* p);
 static int apply_shape(pfs_world* w, int32_t shape, int32_t search);
 
-static uint32_t list_rows_for(const pfs_params& p, uint32_t n, const float* pos4, bool geo) {
+static uint32_t list_rows_for(const pfs_params& p, uint32_t n, const float* pos4) {
     if (n == 0 || !pos4) return NLIST_CAP;
     double lo[3], hi[3];
     for (int a = 0; a < 3; a++) {
@@ -656,7 +657,7 @@ static uint32_t list_rows_for(const pfs_params& p, uint32_t n, const float* pos4
     double vol = 1.0;
     for (int a = 0; a < 3; a++) vol *= std::max(hi[a] - lo[a], (double)p.h);
     const double h = p.h;
-    const double nb = (geo ? 8.0 : 2.0) * (double)n / vol * (4.0 / 3.0) * 3.14159265358979 * h * h * h;
+    const double nb = (few_slots(n) ? 8.0 : 2.0) * (double)n / vol * (4.0 / 3.0) * 3.14159265358979 * h * h * h;
     if (!(nb > NLIST_CAP)) return NLIST_CAP;
     if (nb >= NLIST_CAP_MAX) return NLIST_CAP_MAX;
     return std::min<uint32_t>(((uint32_t)nb + 15u) & ~15u, NLIST_CAP_MAX);
@@ -681,7 +682,7 @@ int pfs_world_create(const pfs_params* p, uint32_t n, const float* pos4, const f
     if (w->flags & PFS_FLAG_IDS) w->flags |= PFS_FLAG_IDS_INTERNAL;
     w->fluid = fluid_volume(*p, n, pos4);
     derive_params(*p, n, &w->dp, -1, w->fluid);
-    w->list_cap = list_rows_for(*p, n, pos4, w->dp.geo != 0);
+    w->list_cap = list_rows_for(*p, n, pos4);
     w->dp.list_cap = w->list_cap;
     {
         // staged block shape from the initial state's particles per cell
