@@ -635,13 +635,20 @@ unsigned cells_grid(K kernel, size_t dyn) {
 // spans many cells of one or two groups of 64 candidates each and sums once, at
 // the end: 24 groups.  A dense scene's 32 particles of one cell share its groups:
 // 16 groups, 352 pairs of ballots, and five thread blocks fit an SM.
+inline CellsLayout cells_layout(uint32_t entries) {
+    return entries > 1024u ? CellsLayout{entries, 352u, 16u} : CellsLayout{entries, 256u, 24u};
+}
+
 template <class F>
 cudaError_t launch_cells(const DevParams& P, const StepBuffers& b, const F& form, cudaStream_t s) {
-    const CellsLayout lay = b.cells_entries > 1024u ? CellsLayout{b.cells_entries, 352u, 16u}
-                                                     : CellsLayout{b.cells_entries, 256u, 24u};
+    const CellsLayout lay = cells_layout(b.cells_entries);
     const size_t dyn = cells_dyn_bytes(lay);
     auto k = b.sr.scenes ? k_density_cells<F, true> : k_density_cells<F, false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    // The limit belongs to the kernel, not to this table: the largest stage's for
+    // every table, so that another thread's world never lowers it between this call
+    // and the launch or the graph's instantiation.  The launch asks for its own size.
+    const size_t most = std::max(cells_dyn_bytes(cells_layout(CELLS_STAGE_MAX)), cells_dyn_bytes(cells_layout(1024u)));
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e != cudaSuccess) return e;
     const unsigned grid = std::max(1u, std::min(cells_grid(k, dyn), P.n));
     k<<<grid, CELLS_THREADS, dyn, s>>>(P, b.sr, form, b.xp, b.skeys, b.order, b.clist, b.cvshift, b.bcount, b.boffset,
