@@ -141,7 +141,7 @@ struct ViewArgs {
     float3 pos, fwd, right, up;
     float half_h, half_w, step;
     float3 ext;  // normalize(extinctionCoefficients)
-    bool skip_empty;  // coefficients positive, densities finite: no transmittance is Inf or NaN
+    bool skip_empty;  // coefficients positive, densities finite and not negative: no transmittance is Inf or NaN
 };
 
 __device__ __forceinline__ float clamp01(float w) {
@@ -485,9 +485,10 @@ cudaError_t launch_volumetric(const DevParams& P, const float* dmap, const int32
     V.half_w = half_w;
     V.step = step;
     V.ext = make_float3(ext[0], ext[1], ext[2]);
-    // a density is at most 27 n m h^2 / volume, a march's sum far less than 1e6 of them
-    V.skip_empty = ext[0] > 0.0f && ext[1] > 0.0f && ext[2] > 0.0f &&
-                   27.0 * P.n * fabs((double)P.m) * P.h * P.h < 1e30 * fabs((double)P.volume);
+    // A density is at most 27 n m h^2 / volume, a march's sum far less than 1e6 of them;
+    // a negative mass makes light that grows, and an empty sample's term Inf * 0.
+    V.skip_empty = ext[0] > 0.0f && ext[1] > 0.0f && ext[2] > 0.0f && P.m >= 0.0f && P.volume > 0.0f &&
+                   27.0 * P.n * (double)P.m * P.h * P.h < 1e30 * (double)P.volume;
     const int3 dd = make_int3(ddims[0], ddims[1], ddims[2]), ld = make_int3(ldims[0], ldims[1], ldims[2]);
     auto k = narrow(dd) && narrow(ld) ? k_volumetric<uint32_t> : k_volumetric<uint64_t>;
     k<<<(unsigned)((n + RENDER_THREADS - 1) / RENDER_THREADS), RENDER_THREADS, 0, s>>>(
