@@ -16,6 +16,7 @@
 #include <thread>
 #include <vector>
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "../../include/pfs.h"
@@ -203,6 +204,7 @@ void fit_spatial_blocks(DevParams* o, uint32_t cap) {
 
 int status_from_cuda(cudaError_t e) {
     if (e == cudaSuccess) return PFS_OK;
+    cudaGetLastError();  // reported here: the next launch's check is not to find it again
     if (e == cudaErrorMemoryAllocation) return PFS_ENOMEM;
     if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return PFS_ENODEV;
     return PFS_ECUDA;
@@ -338,15 +340,37 @@ k_read(uint32_t n, const float4* __restrict__ x, const float4* __restrict__ v, c
     if (density) density[i] = rr[i].x;
 }
 
+// Whether [p, p + bytes) lies in one allocation of the current context.
+bool in_allocation(const void* p, size_t bytes) {
+    typedef CUresult (*RangeFn)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const RangeFn range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<RangeFn>(f);
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+    return range && range(&base, &size, at) == CUDA_SUCCESS && at >= base && bytes <= size && at - base <= size - bytes;
+}
+
 // Whether a buffer (or none) is memory of this device that float4 stores may take.
-bool on_device(const pfs_world* w, const float* p) {
+// One that ends before its bytes do is left to the copies, which the runtime refuses;
+// stores past it would be another buffer's, or fault.
+bool on_device(const pfs_world* w, const float* p, size_t bytes) {
     if (!p) return true;
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeDevice && a.device == w->device && reinterpret_cast<uintptr_t>(p) % 16 == 0;
+    return a.type == cudaMemoryTypeDevice && a.device == w->device && reinterpret_cast<uintptr_t>(p) % 16 == 0 &&
+           in_allocation(p, bytes);
 }
 
 // One substep on the world's stream.  With profiling on, events bracket the
@@ -897,7 +921,7 @@ int pfs_world_read(pfs_world* w, float* pos4, float* vel4, float* density, uint3
     const uint32_t n = w->n;
     const size_t f4 = (size_t)n * 16, u = (size_t)n * 4;
     cudaError_t e = cudaSuccess;
-    if (n > 0 && on_device(w, pos4) && on_device(w, vel4) && on_device(w, density)) {
+    if (n > 0 && on_device(w, pos4, f4) && on_device(w, vel4, f4) && on_device(w, density, u)) {
         k_read<<<grid256(n), 256, 0, w->stream>>>(n, w->b.x, w->b.v, w->b.rr, reinterpret_cast<float4*>(pos4),
                                                   reinterpret_cast<float4*>(vel4), density);
         e = cudaGetLastError();
