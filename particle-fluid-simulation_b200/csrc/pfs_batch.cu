@@ -626,9 +626,13 @@ int pfs_batch_info_get(pfs_batch* B, pfs_batch_info* out) {
     out->max_particles = B->cap_n;
     out->max_scenes = B->cap_s;
     out->device_bytes = B->arena.bytes;
-    bool geo = false;
-    for (const Scene& s : B->scenes) geo = geo || s.dp.geo != 0;
-    out->launches_per_substep = substep_launches(B->n_total ? B->n_total : 1, geo, false);
+    bool geo = false, all = !B->scenes.empty();
+    for (const Scene& s : B->scenes) {
+        geo = geo || s.dp.geo != 0;
+        all = all && s.dp.geo != 0;
+    }
+    geo = geo && B->b.variant >= NBR_LIST;  // the other shapes scan the table
+    out->launches_per_substep = substep_launches(B->n_total ? B->n_total : 1, geo, geo && all, false);
     return PFS_OK;
 }
 

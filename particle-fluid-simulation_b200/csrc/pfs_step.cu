@@ -301,10 +301,11 @@ cudaError_t launch_integrate(const DevParams& P, const StepBuffers& b, cudaStrea
     return cudaGetLastError();
 }
 
-// sort + reorder/bucket (3; a small world 1) + density + force + integrate (+ the
-// two grid-search passes)
-int substep_launches(uint32_t n, bool geo, bool small) {
-    return n == 0 ? 0 : sort_launches(n) + (small ? 4 : 6) + (geo ? 2 : 0);
+// sort + reorder/bucket (3; a small world 1) + density + force + integrate; with the
+// grid search two density passes more, or instead where no table scan is left, and
+// one force pass more
+int substep_launches(uint32_t n, bool geo_any, bool all_geo, bool small) {
+    return n == 0 ? 0 : sort_launches(n) + (small ? 4 : 6) + (geo_any ? (all_geo ? 2 : 3) : 0);
 }
 
 }  // namespace pfs

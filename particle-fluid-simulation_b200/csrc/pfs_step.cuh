@@ -192,8 +192,9 @@ enum { NBR_SIMPLE = 0, NBR_COMPACT = 1, NBR_LIST = 2, NBR_FLAT = 3, NBR_STAGED =
 // Default shape of new worlds and batches (PFS_NBR_VARIANT=simple|slab|list|flat).
 int nbr_variant();
 
-// Launches one substep issues (sort included; geo: grid search in use).
-int substep_launches(uint32_t n, bool geo, bool small);
+// Launches one substep issues (sort included; geo_any, all_geo: some or all particles
+// use the grid search's passes).
+int substep_launches(uint32_t n, bool geo_any, bool all_geo, bool small);
 // The step's density pass runs one warp per slot (pfs_small.cuh), without the
 // spatial order.  SMALL_SLOTS: where the flat walk and its order become faster
 // (reorder, density and force of one substep, dam break and slab: 16,384 slots 40

@@ -1315,7 +1315,9 @@ int pfs_world_stage_times(pfs_world* w, pfs_stage_times* out) {
 }
 
 int pfs_world_launches_per_substep(const pfs_world* w) {
-    return w ? substep_launches(w->n, w->dp.geo != 0, small_world(w->dp, w->b)) : 0;
+    if (!w) return 0;
+    const bool geo = w->dp.geo != 0 && w->b.variant >= NBR_LIST;  // the other shapes scan the table
+    return substep_launches(w->n, geo, geo, small_world(w->dp, w->b));
 }
 
 int pfs_world_debug_substep(pfs_world* w, pfs_debug_substep* o) {
