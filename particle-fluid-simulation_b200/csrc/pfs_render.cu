@@ -10,7 +10,6 @@
 // round-to-nearest operation in the shaders' order, so results equal the
 // oracle's up to expf and powf, whose device and host versions may differ in
 // the last bits.
-#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -25,7 +24,6 @@ constexpr int RENDER_THREADS = 256;
 
 // Trilinear sample of an x-fastest float image of dims (W, H, D) at
 // normalised uvw, with the oracle's term order (pfso_texture3d).
-template <class I>
 __device__ __forceinline__ float tex3d(const float* __restrict__ img, int3 d, float u0, float u1,
                                        float u2) {
     const float uu[3] = {u0, u1, u2};
@@ -43,8 +41,9 @@ __device__ __forceinline__ float tex3d(const float* __restrict__ img, int3 d, fl
         const int32_t k1 = k == INT32_MAX ? k : k + 1;
         i1[a] = min(max(k1, 0), top);
     }
-    const I W = (I)d.x, H = (I)d.y;
-    auto T = [&](int32_t x, int32_t y, int32_t z) { return __ldg(img + (((I)z * H + (I)y) * W + (I)x)); };
+    // (an image has at most 2^31 voxels)
+    const uint32_t W = (uint32_t)d.x, H = (uint32_t)d.y;
+    auto T = [&](int32_t x, int32_t y, int32_t z) { return __ldg(img + (((uint32_t)z * H + (uint32_t)y) * W + (uint32_t)x)); };
     const float a0 = PFS_SUB(1.0f, f[0]), a1 = f[0], b0 = PFS_SUB(1.0f, f[1]), b1 = f[1],
                 c0 = PFS_SUB(1.0f, f[2]), c1 = f[2];
     float r = 0.0f;
@@ -69,16 +68,15 @@ struct BoxSize {
     bool quick;     // div_by serves
 };
 
-// Box sizes of 2^-30 to 2^45 and images of at most 2^16 voxels a side keep div_by's
-// range (pfs_common.cuh) for offsets up to 2^75, down to 2^-75; a smaller quotient is
-// below 2^-45 either way, and lost in the sample's u * side - 0.5.
-BoxSize box_size(const DevParams& P, const int3 a, const int3 b) {
+// Box sizes of 2^-30 to 2^45 keep div_by's range (pfs_common.cuh) for offsets up to
+// 2^75, down to 2^-75; a smaller quotient is below 2^-45 either way, and lost in the
+// sample's u * side - 0.5 (an image has at most 2^16 voxels a side).
+BoxSize box_size(const DevParams& P) {
     BoxSize B;
     B.s = make_float3(P.maxx - P.minx, P.maxy - P.miny, P.maxz - P.minz);
     B.inv = make_float3(1.0f / B.s.x, 1.0f / B.s.y, 1.0f / B.s.z);
     auto fine = [](float v) { return v >= 0x1p-30f && v <= 0x1p45f; };
-    B.quick = fine(B.s.x) && fine(B.s.y) && fine(B.s.z) &&
-              std::max(std::max(a.x, std::max(a.y, a.z)), std::max(b.x, std::max(b.y, b.z))) <= 1 << 16;
+    B.quick = fine(B.s.x) && fine(B.s.y) && fine(B.s.z);
     return B;
 }
 
@@ -114,7 +112,6 @@ __device__ __forceinline__ bool ray_box(const DevParams& P, float3 o, float3 d, 
     return true;
 }
 
-template <class I>
 __global__ void __launch_bounds__(RENDER_THREADS, 4)
 k_light_volume(DevParams P, BoxSize B, const float* __restrict__ dmap, int3 dd, float ls, float3 sun, int3 ld,
                float* __restrict__ out) {
@@ -132,7 +129,7 @@ k_light_volume(DevParams P, BoxSize B, const float* __restrict__ dmap, int3 dd, 
     float acc = 0.0f;
     for (float t = (t0 < 0.0f) ? 0.0f : t0; t < t1; t = PFS_ADD(t, ls)) {
         const float3 u = in_box(P, B, along(c, t, sun));
-        acc = PFS_ADD(acc, PFS_MUL(tex3d<I>(dmap, dd, u.x, u.y, u.z), ls));
+        acc = PFS_ADD(acc, PFS_MUL(tex3d(dmap, dd, u.x, u.y, u.z), ls));
     }
     out[idx] = acc;
 }
@@ -149,7 +146,6 @@ __device__ __forceinline__ float clamp01(float w) {
     return (1.0f < m) ? 1.0f : m;
 }
 
-template <class I>
 __global__ void __launch_bounds__(RENDER_THREADS, 4)
 k_volumetric(DevParams P, BoxSize B, const float* __restrict__ dmap, int3 dd, const float* __restrict__ lvol,
              int3 ld, ViewArgs V, uint32_t width, uint32_t height, float4* __restrict__ rgba) {
@@ -177,13 +173,13 @@ k_volumetric(DevParams P, BoxSize B, const float* __restrict__ dmap, int3 dd, co
         for (float t = PFS_ADD((t0 < 0.0f) ? 0.0f : t0, V.step); t < PFS_SUB(t1, V.step); t = PFS_ADD(t, V.step)) {
             const float3 w = in_box(P, B, along(V.pos, t, d));
             const float w0 = clamp01(w.x), w1 = clamp01(w.y), w2 = clamp01(w.z);
-            const float dens = PFS_MUL(tex3d<I>(dmap, dd, w0, w1, w2), 0.05f);
+            const float dens = PFS_MUL(tex3d(dmap, dd, w0, w1, w2), 0.05f);
             // an empty sample leaves the light and the optical depth as they are (its
             // terms are +0), and most of a box is empty: the light sample and the six
             // exponentials go (300,000-particle scene, 1280 x 720: 0.29 to 0.16 ms)
             if (V.skip_empty && dens == 0.0f) continue;
             view = PFS_ADD(view, PFS_MUL(dens, V.step));
-            const float sun = tex3d<I>(lvol, ld, w0, w1, w2);
+            const float sun = tex3d(lvol, ld, w0, w1, w2);
             float in[3], vt[3];
 #pragma unroll
             for (int a = 0; a < 3; a++) {
@@ -239,25 +235,22 @@ struct RefrMap {
     BoxSize B;
 };
 
-template <class I>
 __device__ __forceinline__ float map_at(const DevParams& P, const RefrMap& M, float3 q) {
     const float3 u = in_box(P, M.B, q);
-    return tex3d<I>(M.img, M.d, u.x, u.y, u.z);
+    return tex3d(M.img, M.d, u.x, u.y, u.z);
 }
 
 // calculateDensityAlongRay (:205-218), intersectVolume padded by +-1e-4.
-template <class I>
 __device__ float refr_density_along(const DevParams& P, const RefrMap& M, float3 o, float3 d, float sstep) {
     float t0, t1;
     if (!ray_box(P, o, d, 1e-4f, -1e-4f, &t0, &t1)) return 0.0f;
     float acc = 0.0f;
     for (float t = PFS_ADD(gmax(t0, 0.0f), sstep); t < PFS_SUB(t1, sstep); t = PFS_ADD(t, sstep))
-        acc = PFS_ADD(acc, PFS_MUL(map_at<I>(P, M, along(o, t, d)), sstep));
+        acc = PFS_ADD(acc, PFS_MUL(map_at(P, M, along(o, t, d)), sstep));
     return acc;
 }
 
 // getSurfaceNormal (:230-260) with calculateClosestFaceNormal (:193-203).
-template <class I>
 __device__ float3 refr_normal(const DevParams& P, const RefrMap& M, float3 pos) {
     const float mn[3] = {P.minx, P.miny, P.minz}, mx[3] = {P.maxx, P.maxy, P.maxz};
     const float pp[3] = {pos.x, pos.y, pos.z}, sz[3] = {M.B.s.x, M.B.s.y, M.B.s.z};
@@ -277,7 +270,7 @@ __device__ float3 refr_normal(const DevParams& P, const RefrMap& M, float3 pos) 
             up[b] = PFS_ADD(uvw[b], a == b ? texel[a] : 0.0f);
             dn[b] = PFS_SUB(uvw[b], a == b ? texel[a] : 0.0f);
         }
-        g[a] = PFS_SUB(tex3d<I>(M.img, M.d, up[0], up[1], up[2]), tex3d<I>(M.img, M.d, dn[0], dn[1], dn[2]));
+        g[a] = PFS_SUB(tex3d(M.img, M.d, up[0], up[1], up[2]), tex3d(M.img, M.d, dn[0], dn[1], dn[2]));
     }
     const float3 vn = normalize3(make_float3(g[0], g[1], g[2]));
     float o[3], local[3], dl[3];
@@ -306,7 +299,6 @@ struct RefrSurface {
 };
 
 // findNextSurface (:277-325).
-template <class I>
 __device__ RefrSurface refr_next_surface(const DevParams& P, const RefrMap& M, const RefrArgs& A, float3 o,
                                          float3 d, bool inside) {
     RefrSurface s;
@@ -320,16 +312,16 @@ __device__ RefrSurface refr_next_surface(const DevParams& P, const RefrMap& M, c
                                 o.y <= P.maxy && o.z <= P.maxz);
     const float t = inside ? 0.0f : gmax(t0, 0.0f);
     o = along(o, PFS_ADD(t, A.step), d);
-    float prev = out_of_fluid ? 0.0f : map_at<I>(P, M, o);
+    float prev = out_of_fluid ? 0.0f : map_at(P, M, o);
     float dens = 0.0f;
     for (float tt = t; tt < t1; tt = PFS_ADD(tt, A.step)) {
         o = along(o, A.step, d);
-        const float density = map_at<I>(P, M, o);
+        const float density = map_at(P, M, o);
         dens = PFS_ADD(dens, PFS_MUL(density, A.step));
         const bool entering = prev < A.threshold && density >= A.threshold;
         const bool exiting = prev >= A.threshold && density < A.threshold;
         if (inside ? exiting : entering) {
-            float3 n = refr_normal<I>(P, M, o);
+            float3 n = refr_normal(P, M, o);
             if (dot3(n, d) > 0.0f) n = make_float3(-n.x, -n.y, -n.z);
             s.pos = o;
             s.normal = n;
@@ -364,7 +356,6 @@ __device__ __forceinline__ float3 offset(float3 p, float3 n, float s) {
 }
 
 // marchRayExpensive (:498-573) for one camera ray.
-template <class I>
 __device__ float3 refr_march(const DevParams& P, const RefrMap& M, const RefrArgs& A, float3 o, float3 d) {
     float tr[3] = {1.0f, 1.0f, 1.0f};
     float light[3] = {0.0f, 0.0f, 0.0f};
@@ -373,7 +364,7 @@ __device__ float3 refr_march(const DevParams& P, const RefrMap& M, const RefrArg
     for (int i = 0; i < A.num_refr; i++) {
         if (isnan(d.x) || isnan(d.y) || isnan(d.z)) return make_float3(1.0f, 0.0f, 1.0f);
         if (PFS_SQRT(dot3(d, d)) < 1e-6f) return make_float3(1.0f, 1.0f, 0.0f);
-        const RefrSurface s = refr_next_surface<I>(P, M, A, o, d, in_fluid);
+        const RefrSurface s = refr_next_surface(P, M, A, o, d, in_fluid);
 #pragma unroll
         for (int a = 0; a < 3; a++) tr[a] = PFS_MUL(tr[a], expf(PFS_MUL(-s.dens, ext[a])));
         if (!s.found) break;
@@ -400,13 +391,13 @@ __device__ float3 refr_march(const DevParams& P, const RefrMap& M, const RefrArg
         if (follow) in_fluid = !in_fluid;
         if (!follow) {
             if (fw > 0.0f) {
-                const float dr = refr_density_along<I>(P, M, fo, fdir, A.light_step);
+                const float dr = refr_density_along(P, M, fo, fdir, A.light_step);
 #pragma unroll
                 for (int a = 0; a < 3; a++)
                     light[a] = PFS_ADD(light[a], PFS_MUL(PFS_MUL(PFS_MUL(1.0f, tr[a]), expf(PFS_MUL(-dr, ext[a]))), fw));
             }
         } else {
-            const float dr = refr_density_along<I>(P, M, ro, rdir, A.light_step);
+            const float dr = refr_density_along(P, M, ro, rdir, A.light_step);
 #pragma unroll
             for (int a = 0; a < 3; a++)
                 light[a] = PFS_ADD(light[a], PFS_MUL(PFS_MUL(PFS_MUL(1.0f, tr[a]), expf(PFS_MUL(-dr, ext[a]))), rw));
@@ -418,7 +409,7 @@ __device__ float3 refr_march(const DevParams& P, const RefrMap& M, const RefrArg
         for (int a = 0; a < 3; a++) tr[a] = PFS_MUL(tr[a], wsel);
         if (gmax(tr[0], gmax(tr[1], tr[2])) < 0.02f) break;
     }
-    const float dr = refr_density_along<I>(P, M, o, d, A.light_step);
+    const float dr = refr_density_along(P, M, o, d, A.light_step);
 #pragma unroll
     for (int a = 0; a < 3; a++)
         light[a] = PFS_ADD(light[a], PFS_MUL(PFS_MUL(1.0f, tr[a]), expf(PFS_MUL(-dr, ext[a]))));
@@ -435,7 +426,6 @@ __device__ float3 refr_march(const DevParams& P, const RefrMap& M, const RefrArg
 // registers: without it the march keeps 80 and takes 204 us, the volumetric one
 // 129; bounds of 6 and 8 blocks there 128 and 141.
 constexpr int REFR_TILE = 16;
-template <class I>
 __global__ void __launch_bounds__(REFR_TILE * REFR_TILE, 1)
 k_refractive(DevParams P, RefrMap M, RefrArgs A, uint32_t width, uint32_t height, float4* __restrict__ rgba) {
     const uint32_t q = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -448,12 +438,9 @@ k_refractive(DevParams P, RefrMap M, RefrArgs A, uint32_t width, uint32_t height
     d.x = PFS_SUB(PFS_SUB(PFS_ADD(PFS_ADD(A.pos.x, A.fwd.x), PFS_MUL(uw, A.right.x)), PFS_MUL(vh, A.up.x)), A.pos.x);
     d.y = PFS_SUB(PFS_SUB(PFS_ADD(PFS_ADD(A.pos.y, A.fwd.y), PFS_MUL(uw, A.right.y)), PFS_MUL(vh, A.up.y)), A.pos.y);
     d.z = PFS_SUB(PFS_SUB(PFS_ADD(PFS_ADD(A.pos.z, A.fwd.z), PFS_MUL(uw, A.right.z)), PFS_MUL(vh, A.up.z)), A.pos.z);
-    const float3 c = refr_march<I>(P, M, A, A.pos, normalize3(d));
+    const float3 c = refr_march(P, M, A, A.pos, normalize3(d));
     rgba[(size_t)y * width + x] = make_float4(c.x, c.y, c.z, 1.0f);
 }
-
-// Whether voxel numbers fit 32 bits.
-bool narrow(const int3 d) { return (uint64_t)d.x * (uint64_t)d.y * (uint64_t)d.z < (1ull << 32); }
 
 }  // namespace
 
@@ -463,9 +450,8 @@ cudaError_t launch_light_volume(const DevParams& P, const float* dmap, const int
     const uint64_t n = (uint64_t)ldims[0] * ldims[1] * ldims[2];
     if (n == 0) return cudaSuccess;
     const int3 dd = make_int3(ddims[0], ddims[1], ddims[2]);
-    auto k = narrow(dd) ? k_light_volume<uint32_t> : k_light_volume<uint64_t>;
-    k<<<(unsigned)((n + RENDER_THREADS - 1) / RENDER_THREADS), RENDER_THREADS, 0, s>>>(
-        P, box_size(P, dd, dd), dmap, dd, light_step, make_float3(sun[0], sun[1], sun[2]),
+    k_light_volume<<<(unsigned)((n + RENDER_THREADS - 1) / RENDER_THREADS), RENDER_THREADS, 0, s>>>(
+        P, box_size(P), dmap, dd, light_step, make_float3(sun[0], sun[1], sun[2]),
         make_int3(ldims[0], ldims[1], ldims[2]), out);
     return cudaGetLastError();
 }
@@ -490,9 +476,8 @@ cudaError_t launch_volumetric(const DevParams& P, const float* dmap, const int32
     V.skip_empty = ext[0] > 0.0f && ext[1] > 0.0f && ext[2] > 0.0f && P.m >= 0.0f && P.volume > 0.0f &&
                    27.0 * P.n * (double)P.m * P.h * P.h < 1e30 * (double)P.volume;
     const int3 dd = make_int3(ddims[0], ddims[1], ddims[2]), ld = make_int3(ldims[0], ldims[1], ldims[2]);
-    auto k = narrow(dd) && narrow(ld) ? k_volumetric<uint32_t> : k_volumetric<uint64_t>;
-    k<<<(unsigned)((n + RENDER_THREADS - 1) / RENDER_THREADS), RENDER_THREADS, 0, s>>>(
-        P, box_size(P, dd, ld), dmap, dd, lvol, ld,
+    k_volumetric<<<(unsigned)((n + RENDER_THREADS - 1) / RENDER_THREADS), RENDER_THREADS, 0, s>>>(
+        P, box_size(P), dmap, dd, lvol, ld,
         V, width, height, reinterpret_cast<float4*>(rgba));
     return cudaGetLastError();
 }
@@ -505,7 +490,7 @@ cudaError_t launch_refractive(const DevParams& P, const float* dmap, const int32
     RefrMap M;
     M.img = dmap;
     M.d = make_int3(ddims[0], ddims[1], ddims[2]);
-    M.B = box_size(P, M.d, M.d);
+    M.B = box_size(P);
     RefrArgs A;
     A.pos = make_float3(cam[0], cam[1], cam[2]);
     A.fwd = make_float3(cam[3], cam[4], cam[5]);
@@ -520,8 +505,7 @@ cudaError_t launch_refractive(const DevParams& P, const float* dmap, const int32
     A.ext = make_float3(ext[0], ext[1], ext[2]);
     A.num_refr = num_refractions;
     const dim3 grid((width + REFR_TILE - 1) / REFR_TILE, (height + REFR_TILE - 1) / REFR_TILE);
-    auto k = narrow(M.d) ? k_refractive<uint32_t> : k_refractive<uint64_t>;
-    k<<<grid, REFR_TILE * REFR_TILE, 0, s>>>(P, M, A, width, height, reinterpret_cast<float4*>(rgba));
+    k_refractive<<<grid, REFR_TILE * REFR_TILE, 0, s>>>(P, M, A, width, height, reinterpret_cast<float4*>(rgba));
     return cudaGetLastError();
 }
 
