@@ -34,6 +34,7 @@ struct DevParams {
     float margin_p, margin_i;
     float rest[6];
     float volume, near_inv, slope_scale, near_slope_scale, r2, skip_d2;
+    uint32_t near_off;  // kn = 0 takes the near pressure away (near_vanishes, pfs_nbr.cuh)
     uint32_t mask;
     uint32_t n;
     int32_t flags;

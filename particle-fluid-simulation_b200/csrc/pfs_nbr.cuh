@@ -216,12 +216,11 @@ __device__ __forceinline__ ForceQuot force_quot(const DevParams& P, float d0, fl
 }
 
 // With kn = 0 (and finite near densities) the near pressure is +-0: its terms
-// leave the sums as they are and are not evaluated.  Unless the kernel's slope at
-// its steepest, (h - d)^2 times the scale, is not finite: 45 / (pi h^6) overflows
-// below h = 5.9e-7, and 0 times it is NaN.
+// leave the sums as they are and are not evaluated.  Unless (near_off) the kernel's
+// slope at its steepest, (h - d)^2 times the scale, is not finite: 45 / (pi h^6)
+// overflows below h = 5.9e-7, and 0 times it is NaN.
 __device__ __forceinline__ bool near_vanishes(const DevParams& P, const ForceSelf& me, float nnd) {
-    return P.kn == 0.0f && me.near_pressure == 0.0f && fabsf(nnd) < INFINITY &&
-           fabsf(PFS_MUL(P.r2, P.near_slope_scale)) < INFINITY;
+    return P.near_off != 0u && me.near_pressure == 0.0f && fabsf(nnd) < INFINITY;
 }
 
 __device__ __forceinline__ void force_term_pre(const DevParams& P, const ForceSelf& me,

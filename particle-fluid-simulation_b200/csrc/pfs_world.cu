@@ -78,6 +78,7 @@ void derive_params(const pfs_params& p, uint32_t n, DevParams* o, int search, do
     o->slope_scale = 15.0f / (PI * powf(h, 5.0f));
     o->near_slope_scale = -45.0f / (PI * powf(h, 6.0f));
     o->r2 = h * h;
+    o->near_off = o->kn == 0.0f && std::isfinite(o->r2 * o->near_slope_scale) ? 1u : 0u;
     float t = h * h;
     while (t > 0.0f && sqrtf(nextafterf(t, 0.0f)) >= h) t = nextafterf(t, 0.0f);
     while (sqrtf(t) < h) t = nextafterf(t, INFINITY);
