@@ -117,7 +117,7 @@ size_t batch_arena_bytes(uint32_t cap_n, uint32_t cap_s, int precision, uint32_t
     size_t b = world_arena_bytes(cap_n, 0, precision, blocks_cap, NLIST_CAP_MAX, 0, precision != PFS_FP16_CELL);
     b += (size_t)cap_s * sizeof(DevParams) + (size_t)cap_n * 4 /*sid*/ + ((size_t)cap_s + 1) * 4;
     b += 2 * (size_t)cap_n * 16; /* x0 v0 */
-    b += ((size_t)blocks_cap / 256 + 1) * 4; /* cvshift */
+    b += ((size_t)blocks_cap / 256 + 1) * sizeof(CellsRule);
     return b + 8 * 256;
 }
 
@@ -131,12 +131,31 @@ DevParams global_params(uint32_t n, uint32_t blocks) {
     return P;
 }
 
+// The scenes' grid search: whether any or all use it, the stage of its cell-grouped
+// density pass, and whether that takes blocks of some scene.
+struct BatchCells {
+    uint32_t geo = 0, all_geo = 1, entries = 0, particles = 0, any = 0;
+    explicit BatchCells(const std::vector<Scene>& scenes) {
+        for (const Scene& s : scenes) {
+            geo |= s.dp.geo;
+            all_geo &= s.dp.geo;
+            if (!s.dp.geo) continue;
+            entries = std::max(entries, cells_entries(s.dp, cell_density(s.dp, s.params, s.n, s.fluid)));
+            particles += s.n;
+        }
+        for (size_t k = 0; k < scenes.size() && !any; k++) any = scenes[k].dp.geo && rule(scenes[k].dp).hi ? 1u : 0u;
+    }
+    CellsRule rule(const DevParams& d) const {
+        return d.geo ? cells_rule(d, entries, particles) : CellsRule{CELLS_TABLE, 0, 0};
+    }
+};
+
 // Re-derive every scene's device parameters for the current packing, upload
 // them, refill the per-slot scene ids and recompute all keys.
 int repack_tables(pfs_batch* B) {
     uint32_t block_base = 0;
-    uint32_t geo_any = 0, all_geo = 1, entries = 0;
-    std::vector<uint32_t> vshift;
+    const BatchCells cells(B->scenes);
+    std::vector<CellsRule> rules;
     std::vector<DevParams> dps(B->scenes.size());
     std::vector<uint32_t> offs(B->scenes.size() + 1);
     for (size_t k = 0; k < B->scenes.size(); k++) {
@@ -147,23 +166,22 @@ int repack_tables(pfs_batch* B) {
         d.block_base = block_base;
         d.list_cap = NLIST_CAP_MAX;
         block_base += (spatial_blocks(d) + kBlockAlign - 1) / kBlockAlign * kBlockAlign;
-        geo_any |= d.geo;
-        all_geo &= d.geo;
-        if (d.geo)
-            entries = std::max(entries, cells_entries(&d, cell_density(d, s.params, s.n, s.fluid)));
-        vshift.resize(block_base / kBlockAlign, d.geo ? (uint32_t)(d.bsx + d.bsy + d.bsz) : 32u);
         dps[k] = d;
         offs[k] = s.off;
     }
+    for (size_t k = 0; k < dps.size(); k++)
+        rules.resize((k + 1 < dps.size() ? dps[k + 1].block_base : block_base) / kBlockAlign, cells.rule(dps[k]));
     offs[B->scenes.size()] = B->n_total;
     if (block_base > B->blocks_cap) return PFS_ERANGE;  // cannot happen: blocks are capped per scene
     B->b.nblocks = block_base;
-    B->b.geo_any = geo_any;
-    B->b.all_geo = all_geo;
-    B->b.cells_entries = entries;
+    B->b.geo_any = cells.geo;
+    B->b.all_geo = cells.all_geo;
+    B->b.cells_entries = cells.entries;
+    B->b.cells_any = cells.any;
     cudaError_t e = cudaSuccess;
-    if (!vshift.empty())
-        e = cudaMemcpyAsync(B->b.cvshift, vshift.data(), vshift.size() * 4, cudaMemcpyHostToDevice, B->stream);
+    if (!rules.empty())
+        e = cudaMemcpyAsync(B->b.crules, rules.data(), rules.size() * sizeof(CellsRule), cudaMemcpyHostToDevice,
+                            B->stream);
     if (e == cudaSuccess && !dps.empty())
         e = cudaMemcpyAsync(B->d_scenes, dps.data(), dps.size() * sizeof(DevParams),
                             cudaMemcpyHostToDevice, B->stream);
@@ -288,7 +306,7 @@ int pfs_batch_create(uint32_t max_particles, uint32_t max_scenes, int32_t precis
     b.scanq = (uint32_t*)a.take(u);
     b.scanq_n = (uint32_t*)a.take(256);
     b.clist = (uint32_t*)a.take(u);
-    b.cvshift = (uint32_t*)a.take(((size_t)B->blocks_cap / 256 + 1) * 4);
+    b.crules = (CellsRule*)a.take(((size_t)B->blocks_cap / 256 + 1) * sizeof(CellsRule));
     B->d_scenes = (DevParams*)a.take((size_t)max_scenes * sizeof(DevParams));
     B->d_sid = (uint32_t*)a.take(u);
     B->d_offs = (uint32_t*)a.take(((size_t)max_scenes + 1) * 4);
@@ -301,7 +319,7 @@ int pfs_batch_create(uint32_t max_particles, uint32_t max_scenes, int32_t precis
     bool ok = (b.fr || precision == PFS_FP16_CELL) && b.x && b.v && b.xs && b.vs && b.xp && b.vp && b.rr && b.keys && b.skeys && b.perm &&
               b.keys_tmp && b.vals_tmp && b.sort_scratch && b.table && b.err && b.order &&
               b.bucket && b.brank && b.bcount && b.boffset && b.bcounter && b.nlist && b.ncount &&
-              b.scanq && b.scanq_n && b.clist && b.cvshift && B->d_scenes && B->d_sid && B->d_offs && B->x0 && B->v0;
+              b.scanq && b.scanq_n && b.clist && b.crules && B->d_scenes && B->d_sid && B->d_offs && B->x0 && B->v0;
     if (ok && precision == PFS_FP16_CELL) ok = fp16_carve(a, max_particles, &B->h16);
     if (!ok) {
         pfs_batch_destroy(B);
@@ -626,13 +644,10 @@ int pfs_batch_info_get(pfs_batch* B, pfs_batch_info* out) {
     out->max_particles = B->cap_n;
     out->max_scenes = B->cap_s;
     out->device_bytes = B->arena.bytes;
-    bool geo = false, all = !B->scenes.empty();
-    for (const Scene& s : B->scenes) {
-        geo = geo || s.dp.geo != 0;
-        all = all && s.dp.geo != 0;
-    }
-    geo = geo && B->b.variant >= NBR_LIST;  // the other shapes scan the table
-    out->launches_per_substep = substep_launches(B->n_total ? B->n_total : 1, geo, geo && all, false);
+    const BatchCells cells(B->scenes);
+    const bool geo = cells.geo && B->b.variant >= NBR_LIST;  // the other shapes scan the table
+    out->launches_per_substep =
+        substep_launches(B->n_total ? B->n_total : 1, geo, geo && cells.all_geo, geo && cells.any, false);
     return PFS_OK;
 }
 

@@ -12,8 +12,8 @@
 // 1.5 here and 0.13 for the particles left; instruction issue binds it, 0.7 of the
 // slots at 94 registers and five blocks on an SM):
 //   1. the spatial order keeps the particles of a block of 2^bsx x 2^bsy x 2^bsz
-//      cells consecutive, cell by cell, about 104 in all; a thread block takes
-//      one such block at a time;
+//      cells consecutive, cell by cell, about 104 in all where the fluid is as
+//      dense as it was created; a thread block takes one such block at a time;
 //   2. the particles of the block's cells and of the layer of cells around them
 //      (three to seven times the block's own) are read once.  Each belongs to
 //      the table slot of its key; those whose slot is one of the slots of these
@@ -32,8 +32,8 @@
 //
 // Left to the one-warp-per-particle pass: particles whose 27 sample cells are not
 // the cells around their own or that lie within rounding of a cell face (edge),
-// blocks whose neighbourhood does not fit even cell by cell and layer by layer,
-// and scenes whose buckets are coarser than cells.
+// blocks for which that pass is faster (cells_rule, pfs_world.cu: they are never
+// listed), and blocks whose neighbourhood does not fit even layer by layer.
 #pragma once
 
 #include <algorithm>
@@ -50,9 +50,6 @@ constexpr int CELLS_THREADS = 128;
 constexpr int CELLS_WARPS = CELLS_THREADS / 32;
 constexpr int CELLS_RUNS = 216;   // a block of 4 x 4 x 4 cells and the layer around it
 constexpr int CELLS_HASH = 512;   // slots of those runs, by open addressing
-// Particles of a block (at most 64 cells) beyond which it is not tried: 128 per
-// cell, and a stage holds one layer of nine such cells.
-constexpr uint32_t CELLS_PILE = 64 * 128;
 constexpr uint32_t CELLS_ALL = (1u << 27) - 1u;  // every sample point in the box
 constexpr uint32_t CELLS_SLOW = 1u << 31;        // meta: left to the one-particle pass
 
@@ -303,7 +300,7 @@ template <class F, bool BATCH>
 __global__ void __launch_bounds__(CELLS_THREADS, 5)
 k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp,
                 const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ order,
-                const uint32_t* __restrict__ clist, const uint32_t* __restrict__ cvshift,
+                const uint32_t* __restrict__ clist, const CellsRule* __restrict__ crules,
                 const uint32_t* __restrict__ bcount, const uint32_t* __restrict__ boffset, CellsLayout lay,
                 float2* __restrict__ rr, float4* __restrict__ fr, int32_t* __restrict__ nlist,
                 int32_t* __restrict__ ncount, uint32_t* __restrict__ scanq, uint32_t* __restrict__ scanq_n,
@@ -327,7 +324,7 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
         if (S.work >= nblk) return;
         const uint32_t id0 = clist[S.work];
         // the block's cells: particles before each, and its segment of the order
-        const uint32_t cells = 1u << (BATCH ? cvshift[id0 >> 8] : (uint32_t)(P0.bsx + P0.bsy + P0.bsz));
+        const uint32_t cells = 1u << (BATCH ? (uint32_t)crules[id0 >> 8].shift : (uint32_t)(P0.bsx + P0.bsy + P0.bsz));
         if (warp == 0) {
             const uint32_t c0 = (uint32_t)lane < cells ? bcount[id0 + lane] : 0u;
             const uint32_t c1 = (uint32_t)lane + 32u < cells ? bcount[id0 + 32 + lane] : 0u;
@@ -354,14 +351,6 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
             if (tid == 0) atomicOr(err, ERR_SORT_COUNT);
             continue;
         }
-        // a pile: nothing of the block fits
-        if (members > CELLS_PILE) {
-            if (tid == 0) S.work = atomicAdd(scanq_n + CTR_SLOW, members);
-            __syncthreads();
-            for (uint32_t k = tid; k < members; k += CELLS_THREADS)
-                if (S.work + k < n) slowq[S.work + k] = seg + k;
-            continue;
-        }
         if constexpr (BATCH) {
             const uint32_t i0 = order[seg];
             if (i0 >= n) {
@@ -374,27 +363,20 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
             __syncthreads();
         }
         const uint32_t lb = (id0 - P.block_base) >> (P.bsx + P.bsy + P.bsz);
-        const int3 dim0 = make_int3(1 << P.bsx, 1 << P.bsy, 1 << P.bsz);
-        const int3 b0 = make_int3((int)(lb % P.nbx) << P.bsx, (int)(lb / P.nbx % P.nby) << P.bsy,
-                                  (int)(lb / (P.nbx * P.nby)) << P.bsz);
+        const int3 dim = make_int3(1 << P.bsx, 1 << P.bsy, 1 << P.bsz);
+        const int3 b = make_int3((int)(lb % P.nbx) << P.bsx, (int)(lb / P.nbx % P.nby) << P.bsy,
+                                 (int)(lb / (P.nbx * P.nby)) << P.bsz);
         const float h = P.h, skip = P.skip_d2;
-        const bool coarse = P.cshift != 0;
-        // pass -1: the whole block, P.blayers layers at a time; if a stage does not
-        // fit, the block's cells one by one and layer by layer (passes 0 ..)
-        int last = coarse || cells == 1u ? -1 : (int)cells - 1;
-        for (int pass = -1; pass <= last; pass++) {
-            const bool whole = pass < 0;
-            const int3 dim = whole ? dim0 : make_int3(1, 1, 1);
-            const int3 b = whole ? b0
-                                 : make_int3(b0.x + (pass & (dim0.x - 1)), b0.y + (pass >> P.bsx & (dim0.y - 1)),
-                                             b0.z + (pass >> (P.bsx + P.bsy)));
-            const uint32_t p_lo = whole ? 0u : S.start[pass], p_hi = whole ? members : S.start[pass + 1];
-            const int layers = dim.z + 2, zs = whole ? min(P.blayers, layers) : 1;
-            bool fits = !coarse, staged = false;
-            for (uint32_t t0 = p_lo; t0 < p_hi; t0 += CELLS_THREADS) {
+        // as many layers at a time as the block's own density fills seven eighths of
+        // the stage with; where that does not fit, one at a time
+        const int layers = dim.z + 2;
+        const float runs = (float)((dim.x + 2) * (dim.y + 2)), density = (float)members / (float)cells;
+        for (int zs = cells_layers(runs, layers, density, (float)(1u << __popc(P.mask)), (float)lay.entries);; zs = 1) {
+            bool fits = true, staged = false;
+            for (uint32_t t0 = 0; t0 < members; t0 += CELLS_THREADS) {
                 // ---- the tile's particles
                 __syncthreads();
-                const uint32_t tile = min(p_hi - t0, (uint32_t)CELLS_THREADS);
+                const uint32_t tile = min(members - t0, (uint32_t)CELLS_THREADS);
                 const uint32_t t = seg + t0 + tid;
                 const bool have = (uint32_t)tid < tile;
                 bool slow = false;
@@ -429,11 +411,11 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
                         const float f = PFS_DIV(PFS_SUB(v, mn), h) - (float)c;
                         return !(f > P.edge && f < 1.0f - P.edge);
                     };
-                    const uint32_t lx = (uint32_t)(cx[1] - b0.x), ly = (uint32_t)(cy[1] - b0.y),
-                                   lz = (uint32_t)(cz[1] - b0.z);
-                    slow = coarse || !listing || lx >= (uint32_t)dim0.x || ly >= (uint32_t)dim0.y ||
-                           lz >= (uint32_t)dim0.z || near_face(sp.x, P.minx, cx[1]) ||
-                           near_face(sp.y, P.miny, cy[1]) || near_face(sp.z, P.minz, cz[1]);
+                    const uint32_t lx = (uint32_t)(cx[1] - b.x), ly = (uint32_t)(cy[1] - b.y),
+                                   lz = (uint32_t)(cz[1] - b.z);
+                    slow = !listing || lx >= (uint32_t)dim.x || ly >= (uint32_t)dim.y || lz >= (uint32_t)dim.z ||
+                           near_face(sp.x, P.minx, cx[1]) || near_face(sp.y, P.miny, cy[1]) ||
+                           near_face(sp.z, P.minz, cz[1]);
                     const uint32_t mx = (vx[0] ? 1u : 0u) | (vx[1] ? 2u : 0u) | (vx[2] ? 4u : 0u);
                     const uint32_t my = (vy[0] ? mx : 0u) | (vy[1] ? mx << 3 : 0u) | (vy[2] ? mx << 6 : 0u);
                     const uint32_t meta = (vz[0] ? my : 0u) | (vz[1] ? my << 9 : 0u) | (vz[2] ? my << 18 : 0u);
@@ -449,13 +431,12 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
                         if (c + s < 64u && S.start[c + s] <= t0 + tid) c += s;
                     S.cell[tid] = c;
                 }
-                // left to the one-particle pass (each once: by the whole-block pass)
+                // left to the one-particle pass
                 auto leave = [&](bool which) {
                     if (!which) return;
                     const uint32_t q = atomicAdd(scanq_n + CTR_SLOW, 1u);
                     if (q < n) slowq[q] = t;
                 };
-                if (whole) leave(slow);
                 __syncthreads();
                 // ---- this warp's share of the tile: an even one, since a warp without
                 // particles would only wait at the next barrier (full warps instead:
@@ -539,8 +520,8 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
                         todo &= ~grp;
                         const uint32_t g = __popc(grp);
                         // the cell's 27 runs, those of these layers
-                        const int lx = whole ? (int)c & (dim0.x - 1) : 0, ly = whole ? (int)c >> P.bsx & (dim0.y - 1) : 0,
-                                  lz = whole ? (int)c >> (P.bsx + P.bsy) : 0;
+                        const int lx = (int)c & (dim.x - 1), ly = (int)c >> P.bsx & (dim.y - 1),
+                                  lz = (int)c >> (P.bsx + P.bsy);
                         uint32_t st = 0, ln = 0;
                         {
                             const int dz = lane * 57 >> 9, dr = lane - 9 * dz, dy = dr * 11 >> 5, dx = dr - 3 * dy;
@@ -602,10 +583,11 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
                     drain();
                 }
                 if (!fits) {
-                    if (whole && cells > 1u && !coarse) continue;  // the cells' passes follow
-                    leave(have && !(S.meta[tid] & CELLS_SLOW));
+                    if (zs > 1) break;  // again, one layer at a time
+                    leave(have);
                     continue;
                 }
+                leave(slow);
                 const bool scan = done && lcnt > lcap;
                 if (done) {
                     put_rr(rr, fr, self, sum.finish(P));
@@ -616,7 +598,7 @@ k_density_cells(DevParams P0, SceneRef sr, F form, const float4* __restrict__ xp
                     if (q < n) scanq[n - 1u - q] = self;
                 }
             }
-            if (whole && fits) break;
+            if (fits || zs == 1) break;
         }
     }
 }
@@ -651,7 +633,7 @@ cudaError_t launch_cells(const DevParams& P, const StepBuffers& b, const F& form
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e != cudaSuccess) return e;
     const unsigned grid = std::max(1u, std::min(cells_grid(k, dyn), P.n));
-    k<<<grid, CELLS_THREADS, dyn, s>>>(P, b.sr, form, b.xp, b.skeys, b.order, b.clist, b.cvshift, b.bcount, b.boffset,
+    k<<<grid, CELLS_THREADS, dyn, s>>>(P, b.sr, form, b.xp, b.skeys, b.order, b.clist, b.crules, b.bcount, b.boffset,
                                        lay, b.rr, b.records(), b.nlist, b.ncount, b.scanq, b.scanq_n, b.keys_tmp, b.err);
     return cudaGetLastError();
 }

@@ -46,10 +46,10 @@ struct DevParams {
     uint32_t ngx, ngy, ngz;
     uint32_t nbx, nby, nbz;
     int32_t cshift, bsx, bsy, bsz;
-    // cell-grouped density pass (pfs_cells.cuh): neighbourhood layers staged at a
-    // time, and the distance from a cell face, in cells, within which rounding
-    // could hide a neighbour two cells away
+    // density map (k_map_cells): neighbourhood layers staged at a time
     int32_t blayers;
+    // cell-grouped density pass (pfs_cells.cuh): the distance from a cell face, in
+    // cells, within which rounding could hide a neighbour two cells away
     float edge;
     // batched scenes: the scene's slice of the shared key space (table slots
     // key_base .. key_base + mask) and of the spatial-order blocks; 0 for a
@@ -141,6 +141,29 @@ constexpr uint32_t CELLS_MAX_GRID = 1u << 16;
 // thread blocks share an SM; more only where one layer of one cell needs it.
 constexpr uint32_t CELLS_STAGE = 1088;
 constexpr uint32_t CELLS_STAGE_MAX = 2048;
+
+// Blocks that the cell-grouped density pass takes: 2^shift buckets with lo to hi
+// particles.
+struct CellsRule {
+    uint16_t shift, lo;
+    uint32_t hi;
+};
+constexpr uint16_t CELLS_TABLE = 0xffff;  // shift: buckets of a table-scan scene
+constexpr uint32_t CELLS_MOST = 8192;     // no block of more is taken
+
+// Candidates of a stage of zs of a neighbourhood's `layers` layers of `runs` cells with
+// d particles each: those layers' own, and of the others those that share a slot of the
+// table with them.
+__host__ __device__ __forceinline__ float cells_stage(float runs, float layers, float zs, float d, float slots) {
+    const float share = zs * runs / slots;
+    return runs * d * (zs + (layers - zs) * (share < 1.0f ? share : 1.0f));
+}
+// As many layers as fill seven eighths of a stage of `entries`; at least one.
+__host__ __device__ __forceinline__ int cells_layers(float runs, int layers, float d, float slots, float entries) {
+    int zs = layers;
+    while (zs > 1 && cells_stage(runs, (float)layers, (float)zs, d, slots) > 0.875f * entries) zs--;
+    return zs;
+}
 
 #define PFS_ADD(a, b) __fadd_rn((a), (b))
 #define PFS_SUB(a, b) __fsub_rn((a), (b))
@@ -258,8 +281,11 @@ double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4);
 // Particles per cell where the fluid is.
 double cell_density(const DevParams& P, const pfs_params& p, uint32_t n, double fluid);
 // Entries the cell-grouped density pass stages at a time for P's blocks at this
-// many particles per cell; sets P->blayers.
-uint32_t cells_entries(DevParams* P, double per_cell);
+// many particles per cell.
+uint32_t cells_entries(const DevParams& P, double per_cell);
+// Blocks the cell-grouped density pass takes, of a table of n grid-search particles
+// in all whose stage holds `entries`.
+CellsRule cells_rule(const DevParams& P, uint32_t entries, uint32_t n);
 // The grid search is possible for this table and box.
 bool grid_search_allowed(const pfs_params& p, uint32_t n);
 // Buckets of the spatial processing order.

@@ -430,7 +430,7 @@ constexpr int GEO16_JCAP = 1024;  // in the force pass, by slot number alone
 // Density pass of the grid-search particles the cell-grouped pass leaves
 // (slowq): same sums in the same order, same list and queue decisions.
 template <bool BATCH>
-__global__ void __launch_bounds__(GEO_WARPS * 32, 6)
+__global__ void __launch_bounds__(GEO_WARPS * 32, BATCH ? 8 : 9)
 k_density16_geo(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const uint4* __restrict__ rec,
                 const int2* __restrict__ table, const uint32_t* __restrict__ order,
                 const uint32_t* __restrict__ bcount, const uint32_t* __restrict__ boffset,
@@ -791,7 +791,7 @@ cudaError_t launch_density_fp16(const DevParams& P, const StepBuffers& b, const 
                                     b.scanq_n, b.err);
     }
     if (b.geo_any) {
-        const cudaError_t e = launch_cells(P, b, Dens16{f.rec}, s);
+        const cudaError_t e = !b.cells_any ? cudaSuccess : launch_cells(P, b, Dens16{f.rec}, s);
         if (e != cudaSuccess) return e;
         auto k = b.sr.scenes ? k_density16_geo<true> : k_density16_geo<false>;
         k<<<geo16_grid(k, P.n), GEO_WARPS * 32, 0, s>>>(P, b.sr, b.xp, f.rec, b.table, b.order, b.bcount, b.boffset,

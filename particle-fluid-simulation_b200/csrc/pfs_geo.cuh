@@ -30,6 +30,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "pfs_common.cuh"
@@ -96,13 +97,14 @@ __device__ __forceinline__ int warp_gather(const DevParams& P, float x, float y,
             if (lane >= s) incl += t;
         }
         const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        // 128 candidates a round, their loads in flight together (a queue holds few
+        // U x 32 candidates a round, their loads in flight together (a queue holds few
         // particles, so a warp's own latency is what the pass takes)
-        for (uint32_t base = 0; base < total; base += 128) {
-            int32_t j[4];
-            bool in[4];
+        auto gather = [&](uint32_t base, auto width) {
+            constexpr int U = decltype(width)::value;
+            int32_t j[U];
+            bool in[U];
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < U; u++) {
                 const uint32_t t = base + 32u * u + (uint32_t)lane;
                 // block of candidate t: the first lane whose inclusive count exceeds t
                 int lo = 0, hi = 31;
@@ -121,7 +123,7 @@ __device__ __forceinline__ int warp_gather(const DevParams& P, float x, float y,
                 j[u] = t < total ? (int32_t)__ldg(order + bo + (t - (bincl - bc))) : -1;
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < U; u++) {
                 if (j[u] >= 0 && (uint32_t)j[u] >= n) {
                     atomicOr(err, ERR_PERM_RANGE);
                     j[u] = -1;
@@ -129,12 +131,19 @@ __device__ __forceinline__ int warp_gather(const DevParams& P, float x, float y,
                 in[u] = j[u] >= 0 && test(j[u]);
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
+            for (int u = 0; u < U; u++) {
                 const uint32_t mask = __ballot_sync(0xffffffffu, in[u]);
                 const int pos = m + __popc(mask & ((1u << lane) - 1u));
                 if (in[u] && pos < cap) s_j[pos] = j[u];
                 m += __popc(mask);
             }
+        };
+        // (a sparse neighbourhood holds a few: 300,000 particles of 2.3 candidates, all
+        // in this pass, 764 us with rounds of 128, 709 with one of 32)
+        if (total <= 32u) {
+            if (total) gather(0u, std::integral_constant<int, 1>{});
+        } else {
+            for (uint32_t base = 0; base < total; base += 128) gather(base, std::integral_constant<int, 4>{});
         }
     }
     __syncwarp();
@@ -167,18 +176,20 @@ __device__ __forceinline__ void warp_sort(int32_t* s_j, int m) {
 }
 
 // Work stealing of the persistent grid-search kernels: a warp takes the next
-// GEO_CHUNK items from a counter the reorder zeroes each substep (lane 0
+// `chunk` items from a counter the reorder zeroes each substep (lane 0
 // adds, the warp shares the result).  Particles of dense scenes cost many
 // times those of sparse ones, so the warps of a batch take work as they free
-// up instead of a fixed stride of it.  One at a time: the queues are short (a
-// few of each thousand particles), and one warp taking four of them in turn was
-// most of the pass (300,000 particles, 85 queued: 0.58 ms).  Called by all 32
-// lanes.
-constexpr uint32_t GEO_CHUNK = 1;
-__device__ __forceinline__ uint32_t warp_take(uint32_t* ctr) {
+// up instead of a fixed stride of it.  Called by all 32 lanes.
+__device__ __forceinline__ uint32_t warp_take(uint32_t* ctr, uint32_t chunk) {
     uint32_t base = 0;
-    if ((threadIdx.x & 31) == 0) base = atomicAdd(ctr, GEO_CHUNK);
+    if ((threadIdx.x & 31) == 0) base = atomicAdd(ctr, chunk);
     return __shfl_sync(0xffffffffu, base, 0);
+}
+// Items of a queue of `total` a warp takes at a time.  A short queue (a few of each
+// thousand particles) one: four in turn were most of the pass (300,000 particles, 85
+// queued: 0.58 ms).  A long one four: the counter is one address for all warps.
+__device__ __forceinline__ uint32_t take_chunk(uint32_t total) {
+    return total > 32u * GEO_WARPS * gridDim.x ? 4u : 1u;
 }
 
 // First position k in a[0, m) with a[k] >= key.

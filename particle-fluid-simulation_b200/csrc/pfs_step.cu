@@ -112,15 +112,18 @@ k_reorder(DevParams P0, SceneRef sr, const uint32_t* __restrict__ skeys, const u
 // segments land in about block-id order (row-major in space) and the
 // neighbour passes, which take positions in order, sweep space coherently:
 // a neighbourhood's data is reused from L2 while it is hot.  With the grid
-// search (clist) the non-empty blocks of 2^vshift consecutive buckets are listed
-// in the same order; a block never spans two thread blocks (256 is a multiple of
-// its size, and a batch's scenes start at multiples of 256).
+// search (clist) the blocks of consecutive buckets that the cell-grouped density
+// pass takes (CellsRule, pfs_common.cuh) are listed in the same order, and the
+// positions of the others' particles are queued for the one-warp-per-particle pass
+// (slowq); a block never spans two thread blocks (256 is a multiple of its size, and
+// a batch's scenes start at multiples of 256).
 __global__ void __launch_bounds__(ELEM_THREADS)
-k_bucket_alloc(uint32_t nblocks, const uint32_t* __restrict__ bcount, uint32_t* __restrict__ boffset,
-               uint32_t* __restrict__ bcounter, uint32_t* __restrict__ clist, uint32_t list_n, uint32_t vshift,
-               const uint32_t* __restrict__ cvshift, uint32_t* __restrict__ nlisted) {
+k_bucket_alloc(uint32_t nblocks, uint32_t n, const uint32_t* __restrict__ bcount, uint32_t* __restrict__ boffset,
+               uint32_t* __restrict__ bcounter, uint32_t* __restrict__ clist, CellsRule rule0,
+               const CellsRule* __restrict__ rules, uint32_t* __restrict__ slowq, uint32_t* __restrict__ counters) {
     __shared__ uint32_t s_warp[ELEM_THREADS / 32], s_incl[ELEM_THREADS], s_live[ELEM_THREADS / 32];
-    __shared__ uint32_t s_base, s_list;
+    __shared__ uint32_t s_slow[ELEM_THREADS / 32];
+    __shared__ uint32_t s_base, s_list, s_queue;
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t c = b < nblocks ? bcount[b] : 0u;
@@ -145,29 +148,48 @@ k_bucket_alloc(uint32_t nblocks, const uint32_t* __restrict__ bcount, uint32_t* 
     const uint32_t before = s_warp[warp] + incl - c;
     if (c) boffset[b] = s_base + before;
     if (!clist) return;
-    const uint32_t vs = cvshift ? cvshift[blockIdx.x] : vshift;
-    if (vs >= 32u) return;  // a table-scan scene's buckets
+    const CellsRule rule = rules ? rules[blockIdx.x] : rule0;
+    if (rule.shift == CELLS_TABLE) return;  // a table-scan scene's buckets
     s_incl[threadIdx.x] = before + c;
     __syncthreads();
-    const uint32_t v = 1u << vs;
-    const bool first = (threadIdx.x & (v - 1u)) == 0u && s_incl[threadIdx.x + v - 1u] > before;
+    // the particles of this bucket's block
+    const uint32_t f = threadIdx.x & ~((1u << rule.shift) - 1u);
+    const uint32_t members = s_incl[f + (1u << rule.shift) - 1u] - (f ? s_incl[f - 1u] : 0u);
+    const bool take = members >= rule.lo && members <= rule.hi;
+    const bool first = take && threadIdx.x == f;
     const uint32_t live = __ballot_sync(0xffffffffu, first);
-    if (lane == 0) s_live[warp] = __popc(live);
+    const uint32_t slow = take ? 0u : c;
+    uint32_t sincl = slow;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, sincl, o);
+        if (lane >= o) sincl += t;
+    }
+    if (lane == 31) {
+        s_live[warp] = __popc(live);
+        s_slow[warp] = sincl;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        uint32_t run = 0;
+        uint32_t run = 0, srun = 0;
         for (int w = 0; w < ELEM_THREADS / 32; w++) {
-            const uint32_t t = s_live[w];
+            const uint32_t t = s_live[w], u = s_slow[w];
             s_live[w] = run;
+            s_slow[w] = srun;
             run += t;
+            srun += u;
         }
-        s_list = run ? atomicAdd(nlisted, run) : 0u;
+        s_list = run ? atomicAdd(counters + CTR_BLOCKS, run) : 0u;
+        s_queue = srun ? atomicAdd(counters + CTR_SLOW, srun) : 0u;
     }
     __syncthreads();
     if (first) {
         const uint32_t k = s_list + s_live[warp] + __popc(live & ((1u << lane) - 1u));
-        if (k < list_n) clist[k] = b;
+        if (k < n) clist[k] = b;
     }
+    const uint32_t q = s_queue + s_slow[warp] + sincl - slow;
+    for (uint32_t k = 0; k < slow; k++)
+        if (q + k < n) slowq[q + k] = s_base + before + k;
 }
 
 // Step 3: place each slot in its block's segment.  The block counters are
@@ -277,8 +299,8 @@ cudaError_t launch_reorder(const DevParams& P, const StepBuffers& b, cudaStream_
         if (e != cudaSuccess) return e;
     } else if (nb > 0) {
         k_bucket_alloc<<<grid_for(nb, ELEM_THREADS), ELEM_THREADS, 0, s>>>(
-            nb, b.bcount, b.boffset, b.bcounter, b.geo_any ? b.clist : nullptr, std::min(nb, P.n),
-            (uint32_t)(P.bsx + P.bsy + P.bsz), b.cvshift, b.scanq_n + CTR_BLOCKS);
+            nb, P.n, b.bcount, b.boffset, b.bcounter, b.geo_any ? b.clist : nullptr, b.cells_rule, b.crules, b.keys_tmp,
+            b.scanq_n);
     }
     k_bucket_scatter<<<g, ELEM_THREADS, 0, s>>>(P.n, nb, b.bucket, b.brank, b.boffset, b.bcount,
                                                 b.geo_any, b.order, b.err);
@@ -302,10 +324,10 @@ cudaError_t launch_integrate(const DevParams& P, const StepBuffers& b, cudaStrea
 }
 
 // sort + reorder/bucket (3; a small world 1) + density + force + integrate; with the
-// grid search two density passes more, or instead where no table scan is left, and
-// one force pass more
-int substep_launches(uint32_t n, bool geo_any, bool all_geo, bool small) {
-    return n == 0 ? 0 : sort_launches(n) + (small ? 4 : 6) + (geo_any ? (all_geo ? 2 : 3) : 0);
+// grid search one force pass more and one density pass, or two with the cell-grouped
+// one, more, or instead where no table scan is left
+int substep_launches(uint32_t n, bool geo_any, bool all_geo, bool cells, bool small) {
+    return n == 0 ? 0 : sort_launches(n) + (small ? 4 : 6) + (geo_any ? (all_geo ? 1 : 2) + (cells ? 1 : 0) : 0);
 }
 
 }  // namespace pfs

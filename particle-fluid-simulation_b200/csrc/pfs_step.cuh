@@ -59,11 +59,13 @@ struct StepBuffers {
     uint32_t* scanq;    // n: positions t whose force pass must scan
     uint32_t* scanq_n;  // CTR_WORDS counters, zeroed by the reorder
     // cell-grouped density pass of the grid search (pfs_cells.cuh): the first
-    // bucket of each non-empty block, log2 of the buckets per block for each 256
-    // buckets (batch; a world's own), and the entries a thread block stages
+    // bucket of each block it takes, the rule for that (a batch: of each 256
+    // buckets, null for a world), and the entries a thread block stages
     uint32_t* clist;    // min(buckets, n)
-    uint32_t* cvshift;  // (buckets + 255) / 256, null for a world
+    CellsRule cells_rule;
+    CellsRule* crules;  // (buckets + 255) / 256
     uint32_t cells_entries;
+    uint32_t cells_any;  // the rule takes blocks of some size
     uint32_t all_geo;   // every particle uses the grid search
     // batch of scenes: per-slot scene parameters (null for one world) and
     // the spatial-order blocks of all scenes together
@@ -193,8 +195,8 @@ enum { NBR_SIMPLE = 0, NBR_COMPACT = 1, NBR_LIST = 2, NBR_FLAT = 3, NBR_STAGED =
 int nbr_variant();
 
 // Launches one substep issues (sort included; geo_any, all_geo: some or all particles
-// use the grid search's passes).
-int substep_launches(uint32_t n, bool geo_any, bool all_geo, bool small);
+// use the grid search's passes; cells: the cell-grouped one among them).
+int substep_launches(uint32_t n, bool geo_any, bool all_geo, bool cells, bool small);
 // The step's density pass runs one warp per slot (pfs_small.cuh), without the
 // spatial order.  SMALL_SLOTS: where the flat walk and its order become faster
 // (reorder, density and force of one substep, dam break and slab: 16,384 slots 40

@@ -104,17 +104,21 @@ void derive_params(const pfs_params& p, uint32_t n, DevParams* o, int search, do
     // 1 + 2^-22 u; twice that, and at least the FP16 record's 2^-11
     const float gmax = (float)std::max(g[0], std::max(g[1], g[2]));
     o->edge = p.precision == PFS_FP16_CELL ? 1.0f / 1024.0f : gmax * (1.0f / 2097152.0f);
+    bool thin = false;
     if (o->geo) {
         // a thread block of the density pass takes one block: 104 particles fill
         // its warps; a small world takes smaller blocks, so that it has a few per SM
         if (members == 0) members = std::min(std::max(n / (3u * 148u), 24u), 104u);
-        const double want = 1.2 * (double)members / cell_density(*o, p, n, fluid);
+        const double density = cell_density(*o, p, n, fluid), want = 1.2 * (double)members / density;
+        thin = 64.0 * density < 10.0;
         const int total = want >= 64.0 ? 6 : want >= 2.0 ? (int)std::floor(std::log2(want)) : 0;
         o->bsx = (total + 2) / 3;
         o->bsy = (total - o->bsx + 1) / 2;
         o->bsz = total - o->bsx - o->bsy;
     }
-    const double cap = o->geo ? std::max(16.0 * (double)n, 65536.0) : std::max(4.0 * (double)n, 4096.0);
+    // (buckets of single cells serve blocks; where the largest block holds too few for
+    // the cell-grouped pass, 4.8M buckets of 300,000 particles only cost 25 us a substep)
+    const double cap = o->geo && !thin ? std::max(16.0 * (double)n, 65536.0) : std::max(4.0 * (double)n, 4096.0);
     set_block_counts(o);
     fit_spatial_blocks(o, (uint32_t)std::min(cap, 4294967295.0));
     o->key_base = 0;
@@ -155,12 +159,53 @@ double cell_density(const DevParams& P, const pfs_params& p, uint32_t n, double 
 
 // As many layers of a block's neighbourhood at a time as CELLS_STAGE entries
 // hold, with an eighth to spare; at least one, of up to CELLS_STAGE_MAX entries.
-uint32_t cells_entries(DevParams* P, double per_cell) {
-    const double layer = 1.125 * ((1 << P->bsx) + 2) * ((1 << P->bsy) + 2) * per_cell;
-    const int layers = (1 << P->bsz) + 2;
-    P->blayers = std::min(std::max((int)((CELLS_STAGE - 64.0) / layer), 1), layers);
-    const double want = std::min(std::max(layer * P->blayers + 64.0, 384.0), (double)CELLS_STAGE_MAX);
+uint32_t cells_entries(const DevParams& P, double per_cell) {
+    const double layer = 1.125 * ((1 << P.bsx) + 2) * ((1 << P.bsy) + 2) * per_cell;
+    const int layers = (1 << P.bsz) + 2;
+    const int at_a_time = std::min(std::max((int)((CELLS_STAGE - 64.0) / layer), 1), layers);
+    const double want = std::min(std::max(layer * at_a_time + 64.0, 384.0), (double)CELLS_STAGE_MAX);
     return ((uint32_t)want + 63u) & ~63u;
+}
+
+// What the two density passes of the grid search take, in ns of the whole device: a
+// block of m particles of the cell-grouped pass (740 thread blocks are resident), and
+// a particle of the one-warp-per-particle pass.  d: particles per cell; the block's
+// neighbourhood of R cells holds R d.  A stage that does not hold the neighbourhood is
+// built again for each 128 particles and each few layers; a run of the table holds, of
+// a table of few slots, particles of all staged cells.  Fitted to measured passes of
+// uniform fluids, 20,000 to 1,000,000 particles, 0.06 to 110 per cell, 8 to 4,096
+// slots, blocks of 1 to 64 cells: the cell-grouped pass within 18% (one deviation), the
+// other within 7%.  So single cells pay from 8 particles up, blocks of 64 from 10, both
+// more in tables of under 100 slots; a fluid that has spread from 97 to 2.6 particles a
+// cell took 3.3 ms in blocks of one cell and takes 0.82 left to the other pass.
+static double cells_block_ns(double m, double d, double R, double builds, double slots) {
+    return 4.8 + builds * (12.1 + 0.019 * R * d) + m * (0.234 + 0.00175 * 27.0 * d + 0.00226 * 27.0 * R * d / slots);
+}
+static double cells_one_ns(double d, double slots) { return 2.2 + 0.171 * d + 0.0018 * 27.0 * d * 27.0 / slots; }
+
+// The blocks taken: those faster so, and none that by itself takes as long as the
+// other pass takes for all n (a block is one thread block's: a small world's few blocks
+// leave most of the device idle; 2,835 particles of a packed world 0.09 against 1.6 ms).
+CellsRule cells_rule(const DevParams& P, uint32_t entries, uint32_t n) {
+    const double cells = (double)(1 << (P.bsx + P.bsy + P.bsz)), slots = (double)(1ull << __builtin_popcount(P.mask));
+    const double runs = (double)((1 << P.bsx) + 2) * (double)((1 << P.bsy) + 2);
+    const int layers = (1 << P.bsz) + 2;
+    CellsRule r{(uint16_t)(P.bsx + P.bsy + P.bsz), 1u, 0u};
+    if (P.cshift) return r;  // buckets coarser than cells
+    for (uint32_t m = 1; m <= CELLS_MOST; m += std::max(1u, m / 32u)) {
+        const double d = m / cells;
+        // (the cells around may hold fewer: this block's count a deviation high)
+        if (cells_stage(runs, layers, 1, d, slots) * (1.0 - 1.0 / std::sqrt((double)m)) > entries) break;
+        const int zs = cells_layers(runs, layers, d, slots, entries);
+        const double builds = zs < layers ? std::ceil((double)layers / zs) * std::ceil(m / 128.0) : 1.0;
+        const double block = cells_block_ns(m, d, runs * layers, builds, slots), one = cells_one_ns(d, slots);
+        const double alone = 8.0 + 0.74 * block, whole = 10.0 + 0.18 * d + 1e-3 * n * one;  // us
+        if (block <= 0.85 * m * one && alone <= 0.6 * whole) {
+            if (!r.hi) r.lo = (uint16_t)m;
+            r.hi = m;
+        }
+    }
+    return r;
 }
 
 double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4) {
@@ -441,7 +486,9 @@ int set_device(pfs_world* w) { return status_from_cuda(cudaSetDevice(w->device))
 // The grid search's flags and staging for the world's current parameters.
 void set_cells(pfs_world* w) {
     w->b.geo_any = w->b.all_geo = w->dp.geo;
-    w->b.cells_entries = cells_entries(&w->dp, cell_density(w->dp, w->params, w->n, w->fluid));
+    w->b.cells_entries = cells_entries(w->dp, cell_density(w->dp, w->params, w->n, w->fluid));
+    w->b.cells_rule = cells_rule(w->dp, w->b.cells_entries, w->n);
+    w->b.cells_any = w->dp.geo && w->b.cells_rule.hi ? 1u : 0u;
 }
 
 int carve(pfs_world* w) {
@@ -489,7 +536,7 @@ int carve(pfs_world* w) {
     b.blist = (uint32_t*)a.take(((size_t)w->staged_blocks + 1) * 4);
     b.st_counters = (uint32_t*)a.take(256);
     b.clist = (uint32_t*)a.take(u);
-    b.cvshift = nullptr;
+    b.crules = nullptr;
     set_cells(w);
     b.fast = w->params.precision == PFS_FP32_FAST ? 1 : 0;
     b.sr = SceneRef{nullptr, nullptr};
@@ -1318,7 +1365,7 @@ int pfs_world_stage_times(pfs_world* w, pfs_stage_times* out) {
 int pfs_world_launches_per_substep(const pfs_world* w) {
     if (!w) return 0;
     const bool geo = w->dp.geo != 0 && w->b.variant >= NBR_LIST;  // the other shapes scan the table
-    return substep_launches(w->n, geo, geo, small_world(w->dp, w->b));
+    return substep_launches(w->n, geo, geo, geo && w->b.cells_any, small_world(w->dp, w->b));
 }
 
 int pfs_world_debug_substep(pfs_world* w, pfs_debug_substep* o) {
