@@ -46,8 +46,6 @@ struct DevParams {
     uint32_t ngx, ngy, ngz;
     uint32_t nbx, nby, nbz;
     int32_t cshift, bsx, bsy, bsz;
-    // density map (k_map_cells): neighbourhood layers staged at a time
-    int32_t blayers;
     // cell-grouped density pass (pfs_cells.cuh): the distance from a cell face, in
     // cells, within which rounding could hide a neighbour two cells away
     float edge;

@@ -12,9 +12,8 @@
 // is rebuilt from its sorted keys for the call (the step's integrate clears it)
 // and cleared again.
 //
-// Where the table has few slots the work is grouped by cell (k_map_cells; elsewhere
-// k_map_flat), as in the density pass of the grid
-// search (pfs_cells.cuh).  One thread per voxel walking its own 27 runs waits on
+// Where the table has few slots the work is grouped by cell (k_map_cells; map_route has
+// the rule), as in the density pass of the grid search (pfs_cells.cuh).  One thread per voxel walking its own 27 runs waits on
 // 27 table look-ups, and reads, where the table has few slots, hundreds of
 // distant particles per run: 5.2 ms for the reference's 300,000 particles (4,096
 // slots) at 917,504 voxels, 0.6 ms in all now.  Here a thread block takes a block of cells, reads
@@ -22,7 +21,8 @@
 // cell, decides what is near), stages what is near in run order and slot order,
 // tests each cell's voxels against 64 staged positions per warp step, and sums a
 // voxel's terms in one lane, in the shader's order.  Voxels outside the box, and
-// voxels of cells whose neighbourhood does not fit the stage, walk their runs.
+// voxels of cells whose neighbourhood does not fit the stage, walk their runs, a thread
+// each (k_density_map), behind it.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -157,8 +157,13 @@ __device__ float map_walk(const DevParams& P, const MapArgs& A, float cxp, float
     return PFS_DIV(PFS_MUL(density, 1.0f), P.volume);
 }
 
-// Beside the cells' pass: the voxels the shader skips (0), and the rest of those
-// whose centre lies outside the box.
+// What k_map_cells writes for a voxel it leaves (no result: theirs are numbers or the
+// one NaN that arithmetic gives).
+constexpr uint32_t MAP_LEFT = 0x7fc5a1e7u;
+
+// A thread per voxel: every voxel (ALL), or, behind the cells' pass, those the shader
+// skips (0), the rest of those whose centre lies outside the box, and those left.
+template <bool ALL>
 __global__ void __launch_bounds__(MAP_THREADS)
 k_density_map(DevParams P, MapArgs A, const float4* __restrict__ x, const int2* __restrict__ table,
               float* __restrict__ out, uint32_t* __restrict__ err) {
@@ -171,7 +176,8 @@ k_density_map(DevParams P, MapArgs A, const float4* __restrict__ x, const int2* 
         return;
     }
     const float cx = map_centre(P.minx, vx, A.cs), cy = map_centre(P.miny, vy, A.cs), cz = map_centre(P.minz, vz, A.cs);
-    if (!map_inside(P, cx, cy, cz)) out[idx] = map_walk(P, A, cx, cy, cz, x, table, err);
+    if (ALL || !map_inside(P, cx, cy, cz) || __float_as_uint(out[idx]) == MAP_LEFT)
+        out[idx] = map_walk(P, A, cx, cy, cz, x, table, err);
 }
 
 // Every voxel, by the flat walk of pfs_flat.cuh (a thread per voxel, the voxels of
@@ -318,11 +324,12 @@ struct MapShared {
 };
 
 // Stage layers [z0, z0 + zs) of the neighbourhood of the cells [b, b + dim):
-// positions near them in run order and slot order.  False when they do not fit.
-__device__ __forceinline__ bool map_build(const DevParams& P, const MapArgs& A, MapShared& S, const CellsLayout& lay,
+// positions near them in run order and slot order.  Returns how many there are; fits:
+// whether the stage holds them.
+__device__ __forceinline__ uint32_t map_build(const DevParams& P, const MapArgs& A, MapShared& S, const CellsLayout& lay,
                                           float4* ent, uint32_t* zone, const int3 b, const int3 dim, int z0, int zs,
                                           const float4* __restrict__ x, const int2* __restrict__ table,
-                                          const uint32_t* __restrict__ code, uint32_t* __restrict__ err) {
+                                          const uint32_t* __restrict__ code, bool& fits, uint32_t* __restrict__ err) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t full = 0xffffffffu, lt = (1u << lane) - 1u;
     const uint32_t n = P.n, zcap = cells_warp_bytes(lay) / 4;
@@ -418,11 +425,12 @@ __device__ __forceinline__ bool map_build(const DevParams& P, const MapArgs& A, 
         total += k;
         most = max(most, k);
     }
-    if (most > zcap || total > lay.entries) return false;
+    fits = most <= zcap && total <= lay.entries;
+    if (!fits) return total;
 #pragma unroll 4
     for (uint32_t k = lane; k < zn; k += 32) ent[base + k] = __ldg(x + zone[k]);
     cells_scan(S.warp_sum, S.off, R);
-    return true;
+    return total;
 }
 
 // Per axis, the first voxel of the cells b + 0 .. b + 7 (the voxel of a cell is
@@ -531,22 +539,25 @@ k_map_cells(DevParams P, MapArgs A, CellsLayout lay, const float4* __restrict__ 
         __syncthreads();
         const uint32_t voxels = S.start[64];
         if (voxels == 0u) continue;
-        // pass -2: the whole block in one stage (most blocks have little near them);
-        // if that does not fit, pass -1: P.blayers layers a stage; if a stage does not
-        // fit, the block's cells one by one, a layer a stage
-        int last = cells == 1 ? -1 : cells - 1;
-        for (int pass = -2; pass <= last; pass++) {
-            const bool whole = pass < 0;
+        // The whole neighbourhood in one stage (most blocks have little near them);
+        // where that does not fit, as many layers as it suggests, and then one.  Then
+        // cell by cell, in the same way, where there are blocks for every thread block
+        // (each of its cells in turn is what a small map waits for: 1,372 voxels 0.6 ms),
+        // and what is left walks.
+        const bool split = cells > 1 && nblk >= gridDim.x;
+        int cell = -1, zs = dim0.z + 2;
+        bool leave = false;
+        for (;;) {
+            const bool whole = cell < 0;
             const int3 dim = whole ? dim0 : make_int3(1, 1, 1);
             const int3 b = whole ? b0
-                                 : make_int3(b0.x + (pass & (dim0.x - 1)), b0.y + (pass >> P.bsx & (dim0.y - 1)),
-                                             b0.z + (pass >> (P.bsx + P.bsy)));
-            const uint32_t p_lo = whole ? 0u : S.start[pass], p_hi = whole ? voxels : S.start[pass + 1];
-            const int layers = dim.z + 2, zs = pass == -2 ? layers : (whole ? min(P.blayers, layers) : 1);
-            if (pass == -1 && zs == layers && cells > 1) continue;  // tried
-            const bool final_try = !whole || (pass == -1 && cells == 1);
-            bool fits = true, staged = false;
-            for (uint32_t t0 = p_lo; t0 < p_hi && (fits || final_try); t0 += CELLS_THREADS) {
+                                 : make_int3(b0.x + (cell & (dim0.x - 1)), b0.y + (cell >> P.bsx & (dim0.y - 1)),
+                                             b0.z + (cell >> (P.bsx + P.bsy)));
+            const uint32_t p_lo = whole ? 0u : S.start[cell], p_hi = whole ? voxels : S.start[cell + 1];
+            const int layers = dim.z + 2;
+            bool fits = !leave, staged = false;
+            uint32_t held = 0;
+            for (uint32_t t0 = p_lo; t0 < p_hi && (fits || leave); t0 += CELLS_THREADS) {
                 // ---- the tile's voxels
                 __syncthreads();
                 const uint32_t tile = min(p_hi - t0, (uint32_t)CELLS_THREADS);
@@ -588,7 +599,8 @@ k_map_cells(DevParams P, MapArgs A, CellsLayout lay, const float4* __restrict__ 
                 const int nx = dim.x + 2, ny = dim.y + 2;
                 for (int z0 = 0; z0 < layers && fits; z0 += zs) {
                     if (!staged || zs < layers)
-                        fits = map_build(P, A, S, lay, ent, zone, b, dim, z0, min(zs, layers - z0), x, table, code, err);
+                        held = map_build(P, A, S, lay, ent, zone, b, dim, z0, min(zs, layers - z0), x, table, code, fits,
+                                         err);
                     if (!fits) break;
                     staged = true;
                     if (w0 >= w1) continue;
@@ -753,27 +765,55 @@ k_map_cells(DevParams P, MapArgs A, CellsLayout lay, const float4* __restrict__ 
                 if (mine_out) {
                     if (fits)
                         out[idx] = PFS_DIV(PFS_MUL(S.nz[tid].x, 1.0f), P.volume);
-                    else if (final_try)
-                        out[idx] = map_walk(P, A, -S.nxy[tid].x, -S.nxy[tid].z, -S.nz[tid].y, x, table, err);
+                    else if (leave)
+                        out[idx] = __uint_as_float(MAP_LEFT);
                 }
             }
-            if (whole && fits) break;
+            if (!fits && !leave) {
+                // (a layer of the middle holds more than the mean)
+                const float fit = 0.85f * (float)lay.entries * (float)zs / (float)held;
+                if (zs > 1 && fit >= 0.7f) {
+                    zs = zs == layers ? min(max((int)fit, 1), layers - 1) : 1;
+                } else if (whole && split) {
+                    cell = 0;
+                    zs = 3;
+                } else {
+                    leave = true;
+                }
+                continue;
+            }
+            if (whole || cell + 1 == cells) break;
+            cell++;
+            zs = 3;
+            leave = false;
         }
     }
 }
 
 }  // namespace
 
+// Positions a layer of a block's neighbourhood holds: its cells' own, and in a table of
+// few slots those of the whole neighbourhood that share a slot with one of them, once
+// for each.
+static double map_layer(int sx, int sy, int sz, double per_cell, double slots) {
+    const double runs = ((1 << sx) + 2.25) * ((1 << sy) + 2.25);
+    return runs * per_cell * (1.0 + runs * ((1 << sz) + 2.25) / slots);
+}
+
 // Cells per block: about 64 voxels (half a tile, for small maps' sake), as many
-// cells as the stage holds at the fluid's density; at most 4 x 4 x 4.
+// cells as the stage holds at the fluid's density, and runs that are mostly of
+// different slots; at most 4 x 4 x 4.
 static void map_blocks(DevParams* P, float cell_size, double per_cell) {
     const double vpc = std::pow((double)P->h / (double)cell_size, 3.0);
+    const double slots = (double)(1ull << __builtin_popcount(P->mask));
     P->cshift = 0;
     P->bsx = P->bsy = P->bsz = 0;
     for (int total = 1; total <= 6; total++) {
         const int sx = (total + 2) / 3, sy = (total - sx + 1) / 2, sz = total - sx - sy;
-        const double layer = ((1 << sx) + 2.25) * ((1 << sy) + 2.25) * per_cell;
-        if (layer > (double)MAP_STAGE || (double)(1 << (total - 1)) * vpc >= 128.0) break;
+        const double runs = (double)((1 << sx) + 2) * ((1 << sy) + 2) * ((1 << sz) + 2);
+        if (map_layer(sx, sy, sz, per_cell, slots) > (double)MAP_STAGE || (double)(1 << (total - 1)) * vpc >= 128.0 ||
+            runs > 1.5 * slots)
+            break;
         P->bsx = sx;
         P->bsy = sy;
         P->bsz = sz;
@@ -783,9 +823,50 @@ static void map_blocks(DevParams* P, float cell_size, double per_cell) {
     P->nbx = (P->ngx >> P->bsx) + 1;
     P->nby = (P->ngy >> P->bsy) + 1;
     P->nbz = (P->ngz >> P->bsz) + 1;
-    const double layer = 1.25 * ((1 << P->bsx) + 2.25) * ((1 << P->bsy) + 2.25) * per_cell;
-    const int layers = (1 << P->bsz) + 2;
-    P->blayers = std::min(std::max((int)(((double)MAP_STAGE - 64.0) / layer), 1), layers);
+}
+
+// Which kernel makes a map: the blocks of cells (M: map_blocks), the flat walk or a thread
+// per voxel: the least of what each takes, in us.  Fitted to the three kernels' times of
+// 2,650 maps (300 to 260,000 particles, 4 to 16,384 slots, 0.3 to 100 particles a cell,
+// 1/37 to 27 voxels a cell, the box 3% to all full; one deviation 40 to 60%); the kernel
+// taken was slower than a thread per voxel by more than 5% in 18 of them, and 0.51 of it
+// in the mean, where the least of the three is 0.48.  So a map of 666 particles on 32 slots,
+// 1,372 voxels, walks (83 us, blocks 610), the reference's 300,000 on 4,096 are grouped
+// (0.6 ms, walks 5.2), a full table's runs, which hold a few entries, are walked flat
+// (1M-particle slab, 1M voxels: 0.25 ms, blocks 0.38, a thread per voxel 0.31), and runs of
+// hundreds a thread per voxel, with twice the flat walk's threads on an SM.
+enum MapRoute { MAP_PLAIN, MAP_FLAT, MAP_CELLS };
+static MapRoute map_route(const DevParams& P, const DevParams& M, const MapArgs& A, double per_cell) {
+    const double n = P.n, slots = (double)(1ull << __builtin_popcount(P.mask));
+    // entries of a run of an empty cell, and of one in the fluid
+    const double run = n / slots, wet_run = run + per_cell;
+    const double thousands = 1e-3 * (double)A.img.x * (double)A.img.y * (double)A.img.z;
+    const double voxels_a_cell = std::pow((double)P.h / (double)A.cs, 3.0);
+    const double wet = std::min(thousands, 1e-3 * n / per_cell * voxels_a_cell), dry = thousands - wet;
+    const double plain = 41.0 + 4.0 * wet_run + dry * (0.12 + 0.0246 * run) + wet * (0.104 + 0.0271 * wet_run);
+    const double flat = 27.5 + 2.72 * wet_run + dry * (0.075 + 0.0349 * run) + wet * (0.071 + 0.0349 * wet_run);
+    // (from here on some runs are more than the flat walk's words, and walked anyway)
+    const MapRoute walk = wet_run <= 32.0 && (run < 4.0 || flat < 0.8 * plain) ? MAP_FLAT : MAP_PLAIN;
+    // the list of blocks takes a sort buffer; and a grid of many more cells than voxels
+    // has little to group
+    const double blocks = (double)M.nbx * M.nby * M.nbz;
+    if (run < 4.0 || std::max(P.ngx, std::max(P.ngy, P.ngz)) > CELLS_MAX_GRID || blocks > std::min(1e3 * thousands, n))
+        return walk;
+    const int layers = (1 << M.bsz) + 2;
+    const double R = (double)((1 << M.bsx) + 2) * ((1 << M.bsy) + 2) * layers;
+    const double layer = map_layer(M.bsx, M.bsy, M.bsz, per_cell, slots), held = layer * layers;
+    if (layer > (double)MAP_STAGE) return walk;  // its voxels would be left
+    const double block_voxels = (double)(1 << (M.bsx + M.bsy + M.bsz)) * voxels_a_cell;
+    const double tiles = std::max(1.0, std::ceil(block_voxels / 128.0));
+    const double scans = 0.9 * held <= 0.95 * MAP_STAGE ? 1.0 : 1.0 + tiles;
+    const double block = 6.9 + scans * (2.5 + 0.00178 * R * wet_run) + 0.0134 * held * tiles +
+                         block_voxels * (0.0138 + 0.00102 * 27.0 * per_cell * (1.0 + R / slots));
+    // blocks that are or lie beside fluid, of 740 resident ones
+    const double side = std::cbrt(n / per_cell) + 2.0;
+    const double near = std::min(blocks, (side / (1 << M.bsx) + 0.5) * (side / (1 << M.bsy) + 0.5) *
+                                             (side / (1 << M.bsz) + 0.5));
+    const double grouped = 37.0 + 0.62e-3 * n + 0.028 * thousands + block * std::max(1.0, near / 757.0);
+    return grouped < 0.8 * (walk == MAP_FLAT ? flat : plain) ? MAP_CELLS : walk;
 }
 
 cudaError_t launch_density_map(const DevParams& P, const StepBuffers& b, float cell_size, double per_cell,
@@ -800,22 +881,15 @@ cudaError_t launch_density_map(const DevParams& P, const StepBuffers& b, float c
         const unsigned gv = (unsigned)((voxels + MAP_THREADS - 1) / MAP_THREADS);
         DevParams M = P;
         map_blocks(&M, cell_size, per_cell);
-        // Where runs hold a few entries the voxels' own walks are faster (1M-particle
-        // slab, full table, 1M voxels: 0.25 ms against 0.38), so the blocks take over
-        // where the grid search does.
-        // (a grid of many more cells than voxels has little to group, and the list of
-        // blocks takes a sort buffer)
-        const double blocks = (double)M.nbx * M.nby * M.nbz;
-        const bool cells = (n >> __builtin_popcount(P.mask)) >= 4u &&
-                           std::max(P.ngx, std::max(P.ngy, P.ngz)) <= CELLS_MAX_GRID &&
-                           blocks <= (double)std::min<uint64_t>(voxels, n);
-        if (!cells) {
+        const MapRoute route = map_route(P, M, A, per_cell);
+        if (route == MAP_PLAIN) {
+            k_density_map<true><<<gv, MAP_THREADS, 0, s>>>(P, A, b.x, b.table, out, b.err);
+        } else if (route == MAP_FLAT) {
             const cudaError_t e = flat_carveout(k_map_flat);
             if (e != cudaSuccess) return e;
             const unsigned gf = (unsigned)((voxels + FLAT_THREADS - 1) / FLAT_THREADS);
             k_map_flat<<<gf, FLAT_THREADS, 0, s>>>(P, A, b.x, b.table, out, b.err);
         } else {
-            k_density_map<<<gv, MAP_THREADS, 0, s>>>(P, A, b.x, b.table, out, b.err);
             // the marks take the neighbour lists' buffer (64 bytes for each 4 x 4 x 4 cells,
             // of which there are at most n)
             const uint32_t coarse = ((P.ngx >> 2) + 1) * ((P.ngy >> 2) + 1) * ((P.ngz >> 2) + 1);
@@ -833,6 +907,7 @@ cudaError_t launch_density_map(const DevParams& P, const StepBuffers& b, float c
             k_map_coarse<<<coarse, CELLS_THREADS, 0, s>>>(M, A, marks, out, b.vals_tmp, listed);
             k_map_cells<<<std::min(cells_grid(k_map_cells, dyn), M.nbx * M.nby * M.nbz), CELLS_THREADS, dyn, s>>>(
                 M, A, lay, b.x, b.table, b.keys_tmp, b.vals_tmp, listed, out, b.err);
+            k_density_map<false><<<gv, MAP_THREADS, 0, s>>>(P, A, b.x, b.table, out, b.err);
         }
     }
     k_table_runs<<<g, MAP_THREADS, 0, s>>>(n, b.skeys, b.table, 0);

@@ -98,7 +98,6 @@ void derive_params(const pfs_params& p, uint32_t n, DevParams* o, int search, do
     o->geo = choose_grid_search(n, g, search) ? 1u : 0u;
     o->cshift = o->geo ? 0 : 1;
     o->bsx = o->bsy = o->bsz = 0;
-    o->blayers = 1;
     // rounding of a cell coordinate u < 2^10: 2^-23 u at most for the two
     // operations together, so neighbours in range differ by less than
     // 1 + 2^-22 u; twice that, and at least the FP16 record's 2^-11
