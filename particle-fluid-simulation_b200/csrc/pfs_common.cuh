@@ -273,8 +273,9 @@ __device__ __forceinline__ float4 speed_color(float3 v) {
 // particles per block to aim for (0: by n).
 void derive_params(const pfs_params& p, uint32_t n, DevParams* out, int search = -1, double fluid = 0.0,
                    uint32_t members = 0);
-// Volume of the bounding box of a sample of an initial state's particles inside
-// the world box (0 for device memory).
+// Volume that an initial state's particles fill, from a sample of them: their bounding
+// box inside the world box, or, where they lie far denser, n over their density there
+// (0: unknown).
 double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4);
 // Particles per cell where the fluid is.
 double cell_density(const DevParams& P, const pfs_params& p, uint32_t n, double fluid);

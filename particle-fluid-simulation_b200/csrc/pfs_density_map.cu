@@ -542,9 +542,10 @@ k_map_cells(DevParams P, MapArgs A, CellsLayout lay, const float4* __restrict__ 
         // The whole neighbourhood in one stage (most blocks have little near them);
         // where that does not fit, as many layers as it suggests, and then one.  Then
         // cell by cell, in the same way, where there are blocks for every thread block
-        // (each of its cells in turn is what a small map waits for: 1,372 voxels 0.6 ms),
-        // and what is left walks.
-        const bool split = cells > 1 && nblk >= gridDim.x;
+        // or a walk takes longer (of a few blocks each one's cells in turn are what the
+        // map waits for, 25 us and more a cell: 1,372 voxels 0.6 ms), and what is left walks.
+        const float run = (float)P.n / (float)(1u << __popc(P.mask));
+        const bool split = cells > 1 && (nblk >= gridDim.x || (float)cells * (25.0f + 0.15f * run) < 4.0f * run);
         int cell = -1, zs = dim0.z + 2;
         bool leave = false;
         for (;;) {

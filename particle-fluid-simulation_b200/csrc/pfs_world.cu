@@ -30,6 +30,25 @@
 
 namespace pfs {
 
+// Whether [p, p + bytes) lies in one allocation of the current context.
+static bool in_allocation(const void* p, size_t bytes) {
+    typedef CUresult (*RangeFn)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const RangeFn range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<RangeFn>(f);
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+    return range && range(&base, &size, at) == CUDA_SUCCESS && at >= base && bytes <= size && at - base <= size - bytes;
+}
+
 // A table of a quarter as many slots as particles or fewer.
 static bool few_slots(uint32_t n) { return n >= 2 && (4ull << __builtin_popcount(n - 1u)) <= (uint64_t)n; }
 
@@ -191,6 +210,8 @@ CellsRule cells_rule(const DevParams& P, uint32_t entries, uint32_t n) {
     const int layers = (1 << P.bsz) + 2;
     CellsRule r{(uint16_t)(P.bsx + P.bsy + P.bsz), 1u, 0u};
     if (P.cshift) return r;  // buckets coarser than cells
+    // every run holds the whole neighbourhood: at 8 slots no size of block was faster
+    if (slots < 32.0) return r;
     for (uint32_t m = 1; m <= CELLS_MOST; m += std::max(1u, m / 32u)) {
         const double d = m / cells;
         // (the cells around may hold fewer: this block's count a deviation high)
@@ -207,18 +228,38 @@ CellsRule cells_rule(const DevParams& P, uint32_t entries, uint32_t n) {
     return r;
 }
 
+// Positions of a sample of an initial state: every n/4096-th of a host array, n/1024-th of
+// device memory (one strided copy; none where the buffer is not one allocation, or for
+// a full table, whose search does not ask).
+static std::vector<float> sample_positions(uint32_t n, const float* pos4) {
+    std::vector<float> out;
+    cudaPointerAttributes attr{};
+    const bool known = cudaPointerGetAttributes(&attr, pos4) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    const bool device = known && attr.type == cudaMemoryTypeDevice;
+    const uint32_t step = std::max(1u, n / (device ? 1024u : 4096u)), count = (n - 1u) / step + 1u;
+    if (device) {
+        if (!few_slots(n) || !in_allocation(pos4, (size_t)n * 16)) return out;
+        out.resize(4 * (size_t)count);
+        if (cudaMemcpy2D(out.data(), 16, pos4, (size_t)step * 16, 16, count, cudaMemcpyDeviceToHost) != cudaSuccess) {
+            cudaGetLastError();
+            out.clear();
+        }
+        return out;
+    }
+    out.resize(4 * (size_t)count);
+    for (uint32_t k = 0; k < count; k++) std::memcpy(&out[4 * (size_t)k], pos4 + 4 * (size_t)k * step, 16);
+    return out;
+}
+
 double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4) {
     if (!pos4 || n == 0) return 0.0;
-    cudaPointerAttributes attr{};
-    if (cudaPointerGetAttributes(&attr, pos4) != cudaSuccess)
-        cudaGetLastError();
-    else if (attr.type == cudaMemoryTypeDevice)
-        return 0.0;
+    const std::vector<float> pos = sample_positions(n, pos4);
+    if (pos.empty()) return 0.0;
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    const uint32_t step = std::max(1u, n / 4096u);
-    for (uint32_t i = 0; i < n; i += step)
+    for (size_t i = 0; i < pos.size(); i += 4)
         for (int a = 0; a < 3; a++) {
-            const double v = pos4[4 * (size_t)i + a];
+            const double v = pos[i + a];
             if (v >= p.box_min[a] && v <= p.box_max[a]) {
                 lo[a] = std::min(lo[a], v);
                 hi[a] = std::max(hi[a], v);
@@ -226,6 +267,31 @@ double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4) {
         }
     double vol = 1.0;
     for (int a = 0; a < 3; a++) vol *= hi[a] >= lo[a] ? std::max(hi[a] - lo[a], (double)p.h) : (double)p.h;
+    // Where the particles lie denser than in their bounding box (several bodies of fluid),
+    // what they lie in: of 1,024 sampled ones (512 of a full table's, of which only the
+    // density map asks), the pairs in one cell.
+    std::vector<uint64_t> cells;
+    const size_t every = std::max<size_t>(1, pos.size() / (few_slots(n) ? 4096u : 2048u));
+    for (size_t i = 0; i < pos.size(); i += 4 * every) {
+        uint64_t key = 0;
+        bool inside = true;
+        for (int a = 0; a < 3; a++) {
+            const double c = std::floor(((double)pos[i + a] - p.box_min[a]) / p.h);
+            inside = inside && c >= 0.0 && c < 2097152.0;
+            key = key << 21 | (inside ? (uint64_t)c : 0u);
+        }
+        if (inside) cells.push_back(key);
+    }
+    std::sort(cells.begin(), cells.end());
+    double pairs = 0.0;
+    for (size_t i = 0, k; i < cells.size(); i = k) {
+        for (k = i; k < cells.size() && cells[k] == cells[i]; k++) {}
+        pairs += (double)(k - i) * (double)(k - i - 1);
+    }
+    if (pairs >= 32.0) {
+        const double m = (double)cells.size(), near = (double)p.h * p.h * p.h * m * (m - 1.0) / pairs;
+        if (near * (1.1 + 3.0 * std::sqrt(2.0 / pairs)) < vol) vol = near;  // (three deviations)
+    }
     return vol;
 }
 
@@ -383,25 +449,6 @@ k_read(uint32_t n, const float4* __restrict__ x, const float4* __restrict__ v, c
     if (pos) pos[i] = x[i];
     if (vel) vel[i] = v[i];
     if (density) density[i] = rr[i].x;
-}
-
-// Whether [p, p + bytes) lies in one allocation of the current context.
-bool in_allocation(const void* p, size_t bytes) {
-    typedef CUresult (*RangeFn)(CUdeviceptr*, size_t*, CUdeviceptr);
-    static const RangeFn range = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess) {
-            cudaGetLastError();
-            f = nullptr;
-        }
-        return reinterpret_cast<RangeFn>(f);
-    }();
-    CUdeviceptr base = 0;
-    size_t size = 0;
-    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
-    return range && range(&base, &size, at) == CUDA_SUCCESS && at >= base && bytes <= size && at - base <= size - bytes;
 }
 
 // Whether a buffer (or none) is memory of this device that float4 stores may take.
