@@ -970,7 +970,7 @@ int nbr_variant() {
 }
 
 bool small_world(const DevParams& P, const StepBuffers& b) {
-    return (b.fp16 || b.variant == NBR_FLAT) && !b.sr.scenes && !P.geo && P.n <= SMALL_SLOTS;
+    return (b.fp16 || b.variant == NBR_FLAT) && !b.sr.scenes && !P.geo && P.n <= SMALL_SLOTS && !b.crowded;
 }
 
 // Launch kernel K in its one-world or batch form.

@@ -71,6 +71,7 @@ struct StepBuffers {
     // the spatial-order blocks of all scenes together
     SceneRef sr;
     uint32_t nblocks;
+    uint32_t crowded;   // too many pairs for pfs_small.cuh
     uint32_t fp16;      // the FP16-cell form
     // FP16-cell form: 16-byte neighbour records the reorder writes (null for
     // the FP32 form)
@@ -200,7 +201,11 @@ int substep_launches(uint32_t n, bool geo_any, bool all_geo, bool cells, bool sm
 // The step's density pass runs one warp per slot (pfs_small.cuh), without the
 // spatial order.  SMALL_SLOTS: where the flat walk and its order become faster
 // (reorder, density and force of one substep, dam break and slab: 16,384 slots 40
-// against 60 us, 32,768 51 against 65, 131,072 160 against 127).
+// against 60 us, 32,768 51 against 65, 131,072 160 against 127).  A warp adds its
+// slot's terms one after another, so of very many the flat walk's lanes are faster
+// (crowded: 16,384 particles that are all each other's neighbours, step of the FP32 form
+// 19.4 against 16.5 ms, FP16 cells 13.7 against 8.6; with 2,000 neighbours each 5.4
+// against 8.6 and 4.0 against 4.8, of 49,151 FP16 particles 6.9 against 6.5).
 constexpr uint32_t SMALL_SLOTS = 49152;
 bool small_world(const DevParams& P, const StepBuffers& b);
 

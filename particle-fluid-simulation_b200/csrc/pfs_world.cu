@@ -529,8 +529,11 @@ int capture_graph(pfs_world* w) {
 
 int set_device(pfs_world* w) { return status_from_cuda(cudaSetDevice(w->device)); }
 
-// The grid search's flags and staging for the world's current parameters.
+// The grid search's flags and staging, and whether a small world is crowded, for the
+// world's current parameters.
 void set_cells(pfs_world* w) {
+    const double pairs = cell_density(w->dp, w->params, w->n, w->fluid) * (double)w->n;
+    w->b.crowded = pairs > (w->params.precision == PFS_FP16_CELL ? 2e7 : 6e7) ? 1u : 0u;
     w->b.geo_any = w->b.all_geo = w->dp.geo;
     w->b.cells_entries = cells_entries(w->dp, cell_density(w->dp, w->params, w->n, w->fluid));
     w->b.cells_rule = cells_rule(w->dp, w->b.cells_entries, w->n);
