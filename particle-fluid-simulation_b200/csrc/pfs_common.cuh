@@ -274,9 +274,9 @@ __device__ __forceinline__ float4 speed_color(float3 v) {
 void derive_params(const pfs_params& p, uint32_t n, DevParams* out, int search = -1, double fluid = 0.0,
                    uint32_t members = 0);
 // Volume that an initial state's particles fill, from a sample of them: their bounding
-// box inside the world box, or, where they lie far denser, n over their density there
-// (0: unknown).
-double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4);
+// box inside the world box (bounding, where the caller has its volume), or, where they
+// lie clearly denser, n over their density there (0: unknown).
+double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4, double bounding = 0.0);
 // Particles per cell where the fluid is.
 double cell_density(const DevParams& P, const pfs_params& p, uint32_t n, double fluid);
 // Entries the cell-grouped density pass stages at a time for P's blocks at this

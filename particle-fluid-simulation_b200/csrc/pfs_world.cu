@@ -228,38 +228,54 @@ CellsRule cells_rule(const DevParams& P, uint32_t entries, uint32_t n) {
     return r;
 }
 
-// Positions of a sample of an initial state: every n/4096-th of a host array, n/1024-th of
-// device memory (one strided copy; none where the buffer is not one allocation, or for
-// a full table, whose search does not ask).
-static std::vector<float> sample_positions(uint32_t n, const float* pos4) {
-    std::vector<float> out;
+static bool is_device_memory(const void* p) {
     cudaPointerAttributes attr{};
-    const bool known = cudaPointerGetAttributes(&attr, pos4) == cudaSuccess;
-    if (!known) cudaGetLastError();
-    const bool device = known && attr.type == cudaMemoryTypeDevice;
-    const uint32_t step = std::max(1u, n / (device ? 1024u : 4096u)), count = (n - 1u) / step + 1u;
-    if (device) {
-        if (!few_slots(n) || !in_allocation(pos4, (size_t)n * 16)) return out;
-        out.resize(4 * (size_t)count);
-        if (cudaMemcpy2D(out.data(), 16, pos4, (size_t)step * 16, 16, count, cudaMemcpyDeviceToHost) != cudaSuccess) {
-            cudaGetLastError();
-            out.clear();
-        }
-        return out;
-    }
-    out.resize(4 * (size_t)count);
-    for (uint32_t k = 0; k < count; k++) std::memcpy(&out[4 * (size_t)k], pos4 + 4 * (size_t)k * step, 16);
-    return out;
+    if (cudaPointerGetAttributes(&attr, p) == cudaSuccess) return attr.type == cudaMemoryTypeDevice;
+    cudaGetLastError();
+    return false;
 }
 
-double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4) {
-    if (!pos4 || n == 0) return 0.0;
-    const std::vector<float> pos = sample_positions(n, pos4);
-    if (pos.empty()) return 0.0;
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (size_t i = 0; i < pos.size(); i += 4)
+// Density of a host array's particles where they are, in particles per cell, from the
+// pairs that share a cell among 512 of them (one at random of each n/512, since those at
+// a fixed distance of a lattice's order lie in a few of its rows).  `box`, their
+// density in their bounding box, where it is not clearly more (by a tenth and three
+// deviations).
+static double paired_density(const pfs_params& p, uint32_t n, const float* pos4, double box) {
+    uint64_t cells[512];
+    const uint32_t count = std::min(512u, n);
+    size_t m = 0;
+    for (uint32_t k = 0; k < count; k++) {
+        const uint32_t lo = (uint32_t)((uint64_t)n * k / count), hi = (uint32_t)((uint64_t)n * (k + 1) / count);
+        uint32_t r = k * 2654435761u;
+        r = (r ^ (r >> 15)) * 0x846ca68bu;
+        const float* x = pos4 + 4 * (size_t)(lo + (r ^ (r >> 16)) % (hi - lo));
+        uint64_t key = 0;
+        bool inside = true;
         for (int a = 0; a < 3; a++) {
-            const double v = pos[i + a];
+            const double c = std::floor(((double)x[a] - p.box_min[a]) / p.h);
+            inside = inside && c >= 0.0 && c < 2097152.0;
+            key = key << 21 | (inside ? (uint64_t)c : 0u);
+        }
+        if (inside) cells[m++] = key;
+    }
+    std::sort(cells, cells + m);
+    double pairs = 0.0;
+    for (size_t i = 0, k; i < m; i = k) {
+        for (k = i; k < m && cells[k] == cells[i]; k++) {}
+        pairs += (double)(k - i) * (double)(k - i - 1);
+    }
+    if (pairs < 32.0) return box;
+    const double d = (double)n * pairs / ((double)m * ((double)m - 1.0));
+    return d > box * (1.1 + 3.0 * std::sqrt(2.0 / pairs)) ? d : box;
+}
+
+// Volume of the bounding box, inside the world box, of every step-th of a host array's
+// particles.
+static double bounding_volume(const pfs_params& p, uint32_t n, const float* pos4, uint32_t step) {
+    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (uint32_t i = 0; i < n; i += step)
+        for (int a = 0; a < 3; a++) {
+            const double v = pos4[4 * (size_t)i + a];
             if (v >= p.box_min[a] && v <= p.box_max[a]) {
                 lo[a] = std::min(lo[a], v);
                 hi[a] = std::max(hi[a], v);
@@ -267,32 +283,28 @@ double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4) {
         }
     double vol = 1.0;
     for (int a = 0; a < 3; a++) vol *= hi[a] >= lo[a] ? std::max(hi[a] - lo[a], (double)p.h) : (double)p.h;
-    // Where the particles lie denser than in their bounding box (several bodies of fluid),
-    // what they lie in: of 1,024 sampled ones (512 of a full table's, of which only the
-    // density map asks), the pairs in one cell.
-    std::vector<uint64_t> cells;
-    const size_t every = std::max<size_t>(1, pos.size() / (few_slots(n) ? 4096u : 2048u));
-    for (size_t i = 0; i < pos.size(); i += 4 * every) {
-        uint64_t key = 0;
-        bool inside = true;
-        for (int a = 0; a < 3; a++) {
-            const double c = std::floor(((double)pos[i + a] - p.box_min[a]) / p.h);
-            inside = inside && c >= 0.0 && c < 2097152.0;
-            key = key << 21 | (inside ? (uint64_t)c : 0u);
-        }
-        if (inside) cells.push_back(key);
-    }
-    std::sort(cells.begin(), cells.end());
-    double pairs = 0.0;
-    for (size_t i = 0, k; i < cells.size(); i = k) {
-        for (k = i; k < cells.size() && cells[k] == cells[i]; k++) {}
-        pairs += (double)(k - i) * (double)(k - i - 1);
-    }
-    if (pairs >= 32.0) {
-        const double m = (double)cells.size(), near = (double)p.h * p.h * p.h * m * (m - 1.0) / pairs;
-        if (near * (1.1 + 3.0 * std::sqrt(2.0 / pairs)) < vol) vol = near;  // (three deviations)
-    }
     return vol;
+}
+
+double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4, double bounding) {
+    if (!pos4 || n == 0) return 0.0;
+    // device memory: every n/1024-th position, in one strided copy; none where the buffer
+    // is not one allocation, or for a full table, whose search does not ask
+    if (is_device_memory(pos4)) {
+        if (!few_slots(n) || !in_allocation(pos4, (size_t)n * 16)) return 0.0;
+        const uint32_t step = std::max(1u, n / 1024u), count = (n - 1u) / step + 1u;
+        float copy[4 * 2048];  // n / 1024 rounded down: fewer than 2,048 rows
+        if (cudaMemcpy2D(copy, 16, pos4, (size_t)step * 16, 16, count, cudaMemcpyDeviceToHost) != cudaSuccess) {
+            cudaGetLastError();
+            return 0.0;
+        }
+        return bounding_volume(p, count, copy, 1);
+    }
+    // denser than in their bounding box (several bodies of fluid; of a full table's only
+    // the density map asks)
+    const double vol = bounding > 0.0 ? bounding : bounding_volume(p, n, pos4, std::max(1u, n / 4096u));
+    const double all = (double)n * p.h * p.h * p.h;
+    return all / paired_density(p, n, pos4, all / vol);
 }
 
 bool grid_search_allowed(const pfs_params& p, uint32_t n) {
@@ -751,32 +763,10 @@ int pfs_version(void) { return 10000; }
 static bool is_device_ptr(const void* p);
 static int apply_shape(pfs_world* w, int32_t shape, int32_t search);
 
-static uint32_t list_rows_for(const pfs_params& p, uint32_t n, const float* pos4) {
-    if (n == 0 || !pos4) return NLIST_CAP;
-    double lo[3], hi[3];
-    for (int a = 0; a < 3; a++) {
-        lo[a] = INFINITY;
-        hi[a] = -INFINITY;
-    }
-    const bool dev = [&] {
-        cudaPointerAttributes attr{};
-        if (cudaPointerGetAttributes(&attr, pos4) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        return attr.type == cudaMemoryTypeDevice;
-    }();
-    if (dev) return NLIST_CAP_MAX;  // device input: no host pass over it
-    for (uint32_t i = 0; i < n; i++)
-        for (int a = 0; a < 3; a++) {
-            const double v = pos4[4 * (size_t)i + a];
-            if (v >= p.box_min[a] && v <= p.box_max[a]) {
-                lo[a] = std::min(lo[a], v);
-                hi[a] = std::max(hi[a], v);
-            }
-        }
-    double vol = 1.0;
-    for (int a = 0; a < 3; a++) vol *= std::max(hi[a] - lo[a], (double)p.h);
+// (vol: 0 for device memory, of which there is no host pass)
+static uint32_t list_rows_for(const pfs_params& p, uint32_t n, double vol) {
+    if (n == 0) return NLIST_CAP;
+    if (!(vol > 0.0)) return NLIST_CAP_MAX;
     const double h = p.h;
     const double nb = (few_slots(n) ? 8.0 : 2.0) * (double)n / vol * (4.0 / 3.0) * 3.14159265358979 * h * h * h;
     if (!(nb > NLIST_CAP)) return NLIST_CAP;
@@ -801,9 +791,10 @@ int pfs_world_create(const pfs_params* p, uint32_t n, const float* pos4, const f
     w->n = n;
     w->flags = p->flags;
     if (w->flags & PFS_FLAG_IDS) w->flags |= PFS_FLAG_IDS_INTERNAL;
-    w->fluid = fluid_volume(*p, n, pos4);
+    const double bounding = is_device_memory(pos4) ? 0.0 : bounding_volume(*p, n, pos4, 1);
+    w->fluid = fluid_volume(*p, n, pos4, bounding);
     derive_params(*p, n, &w->dp, -1, w->fluid);
-    w->list_cap = list_rows_for(*p, n, pos4);
+    w->list_cap = list_rows_for(*p, n, bounding);
     w->dp.list_cap = w->list_cap;
     {
         // staged block shape from the initial state's particles per cell
