@@ -45,7 +45,7 @@ constexpr uint32_t FLAT_LEN_MAX = 127;  // candidates per range word
 // shared-memory words.  As many blocks as fit the largest share (10 of 22 KB)
 // leave the L1 28 KB, where 25% of its sectors hit; 8 blocks of 20 KB leave it
 // 92 KB.  Density pass of 4,194,304 particles in colliding blocks 1,960 -> 970
-// us (FP16 cells 1,085 -> 1,044), of the 1,000,000-particle slab 357 -> 352
+// us (FP16 cells 1,085 -> 1,044), of the 1,048,576-particle slab 357 -> 352
 // (402 -> 400).  Shares of 80% (60 KB of L1): 1,031 and 340 us; 56%: 1,104 and
 // 389 us.
 constexpr int FLAT_CAP = 8;

@@ -251,8 +251,10 @@ k_force_slab(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const flo
 // one listed particle per thread, a block's 128 positions in ascending list
 // length.  PACKED: a neighbour is one 32-byte record (StepBuffers::records has
 // the rule).  Latency binds it: six blocks on an SM (80 registers) and four
-// neighbours in flight; five or seven blocks: 300,000 dense particles 906 and 907
-// us against 815, 1,000,000-particle slab 169 and 156 against 149.
+// neighbours in flight; five or seven blocks: 300,000 dense particles (records) 780 and
+// 780 us against 690, 1,048,576-particle slab 174 and 190 against 157, batches (spilling
+// 40 bytes) of 48 scenes of 16,384 particles 511 and 710 against 505 and of 24 of 40,001
+// 1,335 and 1,349 against 1,210.
 template <bool BATCH, bool FAST, bool PACKED>
 __global__ void __launch_bounds__(NBR_THREADS, 6)
 k_force_list(DevParams P0, SceneRef sr, const float4* __restrict__ xp, const float4* __restrict__ vp,

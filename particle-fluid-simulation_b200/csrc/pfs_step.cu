@@ -187,9 +187,18 @@ k_bucket_alloc(uint32_t nblocks, uint32_t n, const uint32_t* __restrict__ bcount
         const uint32_t k = s_list + s_live[warp] + __popc(live & ((1u << lane) - 1u));
         if (k < n) clist[k] = b;
     }
-    const uint32_t q = s_queue + s_slow[warp] + sincl - slow;
-    for (uint32_t k = 0; k < slow; k++)
-        if (q + k < n) slowq[q + k] = s_base + before + k;
+    // a few positions by the bucket's thread, many (a pile in one cell) by its warp
+    const uint32_t q = s_queue + s_slow[warp] + sincl - slow, t = s_base + before;
+    if (slow <= 32u)
+        for (uint32_t k = 0; k < slow; k++)
+            if (q + k < n) slowq[q + k] = t + k;
+    for (uint32_t many = __ballot_sync(0xffffffffu, slow > 32u); many; many &= many - 1u) {
+        const int src = __ffs(many) - 1;
+        const uint32_t c0 = __shfl_sync(0xffffffffu, slow, src), q0 = __shfl_sync(0xffffffffu, q, src),
+                       t0 = __shfl_sync(0xffffffffu, t, src);
+        for (uint32_t k = lane; k < c0; k += 32)
+            if (q0 + k < n) slowq[q0 + k] = t0 + k;
+    }
 }
 
 // Step 3: place each slot in its block's segment.  The block counters are

@@ -27,7 +27,7 @@ struct StepBuffers {
     // hundreds of neighbours per particle, read as one aligned sector each in
     // place of three parts (300,000 dense particles: force pass 960 -> 815 us for
     // 1 us more in the reorder).  With a full table's tens of neighbours the
-    // record costs what it gives: 1,000,000-particle slab 157 -> 149 us and 9 us
+    // record costs what it gives: 1,048,576-particle slab 157 -> 149 us and 9 us
     // more in the reorder; 4,194,304 particles 434 -> 432 and 55 us more.
     float4* records() const { return all_geo ? fr : nullptr; }
     uint32_t* keys;     // keys of the state positions (next sort's input)

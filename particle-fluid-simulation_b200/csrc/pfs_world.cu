@@ -760,7 +760,7 @@ int pfs_version(void) { return 10000; }
 // Neighbour-list rows of a new world: twice the mean neighbour count (eight times where
 // the table has few slots: there a particle without a list costs a gather by a whole
 // warp, and 150,000 dense particles that fall on each other spent 0.9 ms a substep
-// on them; elsewhere rows only cost memory, 9 ms of a 1,000,000-particle world's
+// on them; elsewhere rows only cost memory, 9 ms of a 1,048,576-particle world's
 // creation) of its initial state (particles in their bounding box, clipped to the world box,
 // times the volume of a sphere of radius h), rounded up to 16 and kept within
 // [NLIST_CAP, NLIST_CAP_MAX].  Particles of denser regions than that fall back
