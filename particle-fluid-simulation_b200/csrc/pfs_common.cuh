@@ -275,8 +275,10 @@ void derive_params(const pfs_params& p, uint32_t n, DevParams* out, int search =
                    uint32_t members = 0);
 // Volume that an initial state's particles fill, from a sample of them: their bounding
 // box inside the world box (bounding, where the caller has its volume), or, where they
-// lie clearly denser, n over their density there (0: unknown).
-double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4, double bounding = 0.0);
+// lie clearly denser, n over their density there (0: unknown, as for device memory
+// without a stream to sample it on and wait for).
+double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4, double bounding = 0.0,
+                    cudaStream_t stream = nullptr);
 // Particles per cell where the fluid is.
 double cell_density(const DevParams& P, const pfs_params& p, uint32_t n, double fluid);
 // Entries the cell-grouped density pass stages at a time for P's blocks at this

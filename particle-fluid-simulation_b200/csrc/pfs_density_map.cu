@@ -480,10 +480,12 @@ k_map_coarse(DevParams P, MapArgs A, const uint8_t* __restrict__ marks, float* _
     }
     map_first(P, A, b, s_first);
     __syncthreads();
-    const int wx = s_first[0][4] - s_first[0][0], wy = s_first[1][4] - s_first[1][0],
-              wz = s_first[2][4] - s_first[2][0];
-    for (int k = tid; k < wx * wy * wz; k += CELLS_THREADS) {
-        const int vx = s_first[0][0] + k % wx, vy = s_first[1][0] + k / wx % wy, vz = s_first[2][0] + k / (wx * wy);
+    // (a map may have 2^31 voxels, and a block all of them)
+    const uint32_t wx = s_first[0][4] - s_first[0][0], wy = s_first[1][4] - s_first[1][0],
+                   wz = s_first[2][4] - s_first[2][0];
+    for (uint32_t k = tid; k < wx * wy * wz; k += CELLS_THREADS) {
+        const int vx = s_first[0][0] + (int)(k % wx), vy = s_first[1][0] + (int)(k / wx % wy),
+                  vz = s_first[2][0] + (int)(k / (wx * wy));
         if (map_out(vx, vy, vz, A.bound) ||
             !map_inside(P, map_centre(P.minx, vx, A.cs), map_centre(P.miny, vy, A.cs), map_centre(P.minz, vz, A.cs)))
             continue;  // k_density_map's

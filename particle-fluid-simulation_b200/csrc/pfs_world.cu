@@ -286,15 +286,19 @@ static double bounding_volume(const pfs_params& p, uint32_t n, const float* pos4
     return vol;
 }
 
-double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4, double bounding) {
+double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4, double bounding, cudaStream_t stream) {
     if (!pos4 || n == 0) return 0.0;
-    // device memory: every n/1024-th position, in one strided copy; none where the buffer
-    // is not one allocation, or for a full table, whose search does not ask
+    // device memory: every n/1024-th position, in one strided copy; none without a stream
+    // to wait for, where the buffer is not one allocation, or for a full table, whose
+    // search does not ask
     if (is_device_memory(pos4)) {
-        if (!few_slots(n) || !in_allocation(pos4, (size_t)n * 16)) return 0.0;
+        if (!stream || !few_slots(n) || !in_allocation(pos4, (size_t)n * 16)) return 0.0;
         const uint32_t step = std::max(1u, n / 1024u), count = (n - 1u) / step + 1u;
         float copy[4 * 2048];  // n / 1024 rounded down: fewer than 2,048 rows
-        if (cudaMemcpy2D(copy, 16, pos4, (size_t)step * 16, 16, count, cudaMemcpyDeviceToHost) != cudaSuccess) {
+        cudaError_t e =
+            cudaMemcpy2DAsync(copy, 16, pos4, (size_t)step * 16, 16, count, cudaMemcpyDeviceToHost, stream);
+        const cudaError_t waited = cudaStreamSynchronize(stream);  // (copy is written until then)
+        if (e != cudaSuccess || waited != cudaSuccess) {
             cudaGetLastError();
             return 0.0;
         }
@@ -797,7 +801,12 @@ int pfs_world_create(const pfs_params* p, uint32_t n, const float* pos4, const f
     w->flags = p->flags;
     if (w->flags & PFS_FLAG_IDS) w->flags |= PFS_FLAG_IDS_INTERNAL;
     const double bounding = is_device_memory(pos4) ? 0.0 : bounding_volume(*p, n, pos4, 1);
-    w->fluid = fluid_volume(*p, n, pos4, bounding);
+    cudaError_t e = cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking);
+    if (e != cudaSuccess) {
+        delete w;
+        return status_from_cuda(e);
+    }
+    w->fluid = fluid_volume(*p, n, pos4, bounding, w->stream);
     derive_params(*p, n, &w->dp, -1, w->fluid);
     w->list_cap = list_rows_for(*p, n, bounding);
     w->dp.list_cap = w->list_cap;
@@ -814,11 +823,6 @@ int pfs_world_create(const pfs_params* p, uint32_t n, const float* pos4, const f
                                         8ull * n + 65536ull);
         w->staged_cfg.staged = w->staged_ok ? 1u : 0u;
         w->staged_blocks = w->staged_ok ? w->staged_cfg.nsx * w->staged_cfg.nsy * w->staged_cfg.nsz : 0u;
-    }
-    cudaError_t e = cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking);
-    if (e != cudaSuccess) {
-        delete w;
-        return status_from_cuda(e);
     }
     rc = carve(w);
     if (rc == PFS_OK) {
