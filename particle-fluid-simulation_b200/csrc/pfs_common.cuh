@@ -273,10 +273,10 @@ __device__ __forceinline__ float4 speed_color(float3 v) {
 // particles per block to aim for (0: by n).
 void derive_params(const pfs_params& p, uint32_t n, DevParams* out, int search = -1, double fluid = 0.0,
                    uint32_t members = 0);
-// Volume that an initial state's particles fill, from a sample of them: their bounding
-// box inside the world box (bounding, where the caller has its volume), or, where they
-// lie clearly denser, n over their density there (0: unknown, as for device memory
-// without a stream to sample it on and wait for).
+// Volume that an initial state's particles fill: their bounding box inside the world box
+// (bounding, where the caller has its volume, else of a sample), or, with `bounding`,
+// where they lie clearly denser, n over their density there (0: unknown, as for device
+// memory without a stream to sample it on and wait for, and full tables' scenes).
 double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4, double bounding = 0.0,
                     cudaStream_t stream = nullptr);
 // Particles per cell where the fluid is.

@@ -304,11 +304,13 @@ double fluid_volume(const pfs_params& p, uint32_t n, const float* pos4, double b
         }
         return bounding_volume(p, count, copy, 1);
     }
+    // a batch's scene: the sample is what adding it costs (80 us a scene with 4,096 positions
+    // and the pairs, 10 so)
+    if (!(bounding > 0.0)) return few_slots(n) ? bounding_volume(p, n, pos4, std::max(1u, n / 1024u)) : 0.0;
     // denser than in their bounding box (several bodies of fluid; of a full table's only
     // the density map asks)
-    const double vol = bounding > 0.0 ? bounding : bounding_volume(p, n, pos4, std::max(1u, n / 4096u));
     const double all = (double)n * p.h * p.h * p.h;
-    return all / paired_density(p, n, pos4, all / vol);
+    return all / paired_density(p, n, pos4, all / bounding);
 }
 
 bool grid_search_allowed(const pfs_params& p, uint32_t n) {
